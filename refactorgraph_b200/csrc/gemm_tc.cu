@@ -30,6 +30,7 @@ static __device__ int s_tc_index_error;// a cache-append position or block-table
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;// 64 x 2 B = one 128-byte swizzle row
 constexpr int TC_THREADS = 192;
+constexpr uint32_t TC_MN_BLOCK = 64 * TC_BK * 2;// one box of an MN-major operand: 64 columns x 64 k-rows
 
 struct TcArgs {
     void *Y;
@@ -145,11 +146,18 @@ struct TcWalk {
 // the accumulator and its epilogue warps store them.  Per SM and k-block that is 32 KiB from L2 instead of 48 for the same 128 x 256
 // outputs: the single-CTA kernel is bound by requests to L2 (ncu: 68 % of request cycles, tensor pipe 80 %; an extra L2 prefetch
 // per box made it 22 % slower).  No load is multicast.
-template<class T, int BN, int STAGES, bool PUSH = false, bool PAIR = false>// PUSH: the epilogue that stores into the all-reduce slots is compiled in
+//
+// MN: the weight matrix is stored [k, out] (MatMul with transB = 0, as exporters write it): its tile is loaded as boxes of 64 output
+// columns x 64 k-rows, one 8 KiB block per 64 columns, and enters the instruction as an MN-major operand (the M side of the skinny
+// forms, the N side otherwise).  A K step of 16 is then 16 rows = 2 KiB further inside each block; the next 64 columns are one
+// block further (leading offset), the next 8 rows 1 KiB further (stride offset).  Nothing is transposed in memory.  These products ran
+// on the CUDA cores before: a two-layer 7B decoder on a 300-token prompt, fp16, all weights [k, out], 11.3 ms then, 0.81 ms now.
+template<class T, int BN, int STAGES, bool PUSH = false, bool PAIR = false, bool MN = false>// PUSH: the epilogue that stores into the all-reduce slots is compiled in
 __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                                               const __grid_constant__ CUtensorMap tmap_b, const TcArgs a) {
     constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, B_BYTES = (PAIR ? BN / 2 : BN) * TC_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr uint32_t ROWS = PAIR ? 2 * TC_BM : TC_BM;// rows of a tile
+    constexpr bool MN_A = MN && BN <= 64, MN_B = MN && BN > 64;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;// 0 = the CTA that issues the products
     const uint32_t unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -201,7 +209,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             uint32_t it = 0, pre = 0;
             // B tile of column tile nt: BN consecutive rows of B, or (SiLU-gate form) 128 gate rows and their 128 up rows
             auto load_b = [&](uint8_t *dst, uint32_t kb, uint32_t nt, uint64_t *bar) {
-                if (BN == 256 && a.swiglu) {
+                if constexpr (MN_B) {
+#pragma unroll
+                    for (uint32_t c = 0; c < BN / 64; ++c) tma_load_2d(dst + c * TC_MN_BLOCK, &tmap_b, nt * BN + c * 64, kb * TC_BK, bar);
+                } else if (BN == 256 && a.swiglu) {
                     tma_load_2d(dst, &tmap_b, kb * TC_BK, nt * 128, bar);
                     tma_load_2d(dst + 128 * TC_BK * 2, &tmap_b, kb * TC_BK, a.swiglu + nt * 128, bar);
                 } else {
@@ -211,7 +222,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             // A tile of row tile mt: 128 consecutive rows of A, or (SiLU-gate form with the weights on the A side) 64 gate rows
             // and their 64 up rows: two boxes of a 64-row tensor map, one behind the other
             auto load_a = [&](uint8_t *dst, uint32_t kb, uint32_t mt, uint64_t *bar) {
-                if (BN <= 64 && a.swiglu) {
+                if constexpr (MN_A) {
+#pragma unroll
+                    for (uint32_t c = 0; c < TC_BM / 64; ++c) tma_load_2d(dst + c * TC_MN_BLOCK, &tmap_a, mt * TC_BM + c * 64, kb * TC_BK, bar);
+                } else if (BN <= 64 && a.swiglu) {
                     tma_load_2d(dst, &tmap_a, kb * TC_BK, mt * 64, bar);
                     tma_load_2d(dst + 64 * TC_BK * 2, &tmap_a, kb * TC_BK, a.swiglu + mt * 64, bar);
                 } else {
@@ -261,7 +275,13 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                         if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * STAGE_BYTES);
                         tma_load_2d_pair(st, &tmap_a, kb * TC_BK, (mt * 2 + rank) * TC_BM, bar);
                         const uint32_t brow = a.swiglu ? (rank ? a.swiglu + nt * 128 : nt * 128) : nt * BN + rank * (BN / 2);
-                        tma_load_2d_pair(st + A_BYTES, &tmap_b, kb * TC_BK, brow, bar);
+                        if constexpr (MN_B) {
+#pragma unroll
+                            for (uint32_t c = 0; c < BN / 128; ++c)
+                                tma_load_2d_pair(st + A_BYTES + c * TC_MN_BLOCK, &tmap_b, brow + c * 64, kb * TC_BK, bar);
+                        } else {
+                            tma_load_2d_pair(st + A_BYTES, &tmap_b, kb * TC_BK, brow, bar);
+                        }
                         continue;
                     }
                     mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
@@ -272,7 +292,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         }
     } else if (warp == 5) {
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = instr_desc(a.is_bf16, ROWS, BN);
+            const uint32_t idesc = instr_desc(a.is_bf16, ROWS, BN) | (MN_A ? 1u << 15 : 0u) | (MN_B ? 1u << 16 : 0u);
             uint32_t it = 0, local = 0;
             bool ok = true;
             TcWalk walk;
@@ -297,7 +317,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES), b_addr = a_addr + A_BYTES;
 #pragma unroll
                     for (int kk = 0; kk < TC_BK / 16; ++kk) {
-                        const uint64_t ad = smem_desc_sw128(a_addr + kk * 32), bd = smem_desc_sw128(b_addr + kk * 32);
+                        const uint64_t ad = MN_A ? smem_desc_sw128_mn(a_addr + kk * 2048, TC_MN_BLOCK) : smem_desc_sw128(a_addr + kk * 32);
+                        const uint64_t bd = MN_B ? smem_desc_sw128_mn(b_addr + kk * 2048, TC_MN_BLOCK) : smem_desc_sw128(b_addr + kk * 32);
                         if constexpr (PAIR) tc_mma_f16_pair(d_tmem, ad, bd, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
                         else
                             tc_mma_f16(d_tmem, ad, bd, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
@@ -777,9 +798,28 @@ bool tma_encode_rows_by_blocks(void *map, const void *base, int is_bf16, uint64_
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A weight matrix stored [k, n] as the kernel's MN-major operand: boxes of 64 columns x 64 k-rows
+static bool make_map_mn(CUtensorMap *map, const void *base, int is_bf16, uint64_t k, uint64_t n) {
+    EncodeFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {n, k};
+    const cuuint64_t strides[1] = {n * 2};
+    const cuuint32_t box[2] = {64, TC_BK};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims,
+              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool gemm_tc_supported(const rg_mat_mul_params *p, const void *const *in, void *const *out) {
     if (p->dtype != RG_FP16 && p->dtype != RG_BF16) return false;
-    if (p->trans_a || !p->trans_b) return false;
+    if (p->trans_a) return false;
+    if (!p->trans_b) {
+        if (p->n % 8 != 0) return false;// rows of an MN-major B start on 16 bytes
+        // a batch is one launch per matrix here and one launch altogether on the CUDA cores (~15 TFLOP/s), which keep the batches of
+        // products that would take them less than about 9 us each
+        if (p->batch > 1 && static_cast<uint64_t>(p->m) * p->n * p->k < (1ull << 26)) return false;
+    }
     if (p->k % 8 != 0 || p->k < 64) return false;
     if (!aligned16(in[0]) || !aligned16(in[1]) || !aligned16(out[0])) return false;
     if (p->batch > 1 && ((p->stride_a % 8) || (p->stride_b % 8) || (p->stride_y % 8))) return false;
@@ -870,12 +910,12 @@ size_t gemm_tc_workspace(const rg_mat_mul_params *p) {
 // waits for a free stage 41 % of the time.  Leaving the activation-tile loads out altogether (timing only): 41.3 us.  What is
 // left is the fill and drain of the memory pipeline around the dependency on the previous kernel (~10 us per launch): the
 // TMA-only stream has no such dependency, so its launches overlap.
-template<class T, int BN, int STAGES, bool PUSH = false>
+template<class T, int BN, int STAGES, bool PUSH = false, bool MN = false>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &a_in, cudaStream_t st) {
     TcArgs a = a_in;
     a.group_m = TC_GROUP_M;
     constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
-    auto kern = gemm_tc_kernel<T, BN, STAGES, PUSH>;
+    auto kern = gemm_tc_kernel<T, BN, STAGES, PUSH, false, MN>;
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     // the whole shared-memory carve-out, so that a CTA of the next kernel can sit beside one of this kernel when both fit
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, static_cast<int>(cudaSharedmemCarveoutMaxShared)));
@@ -893,13 +933,13 @@ static bool tc_pair_enabled() {
     static const bool on = !(std::getenv("RG_B200_GEMM_PAIR") && std::getenv("RG_B200_GEMM_PAIR")[0] == '0');
     return on;
 }
-template<class T>
+template<class T, bool MN = false>
 static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &a_in, cudaStream_t st) {
     constexpr int BN = 256, STAGES = 6;
     TcArgs a = a_in;
     a.group_m = TC_GROUP_M;// of 256-row tiles; measured on 8192 x 12288 x 4096: 4 / 8 / 16 / 32 row tiles per group 577 / 557 / 550 / 605 us
     constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + (BN / 2) * TC_BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
-    auto kern = gemm_tc_kernel<T, BN, STAGES, false, true>;
+    auto kern = gemm_tc_kernel<T, BN, STAGES, false, true, MN>;
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const uint32_t items = ((a.n + BN - 1) / BN) * ((a.m + 2 * TC_BM - 1) / (2 * TC_BM));
     // as many pairs as the device can hold at once (asked once per device; half the SM count where the question fails)
@@ -932,6 +972,10 @@ int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *c
     const size_t es = 2;
     const TcPlan pl = tc_plan(p);
     if (pl.splits > 1 && !ws) return RG_ERR_NULL;
+    const bool mn = !p->trans_b;
+    auto map_b = [&](CUtensorMap *map, const void *base, uint32_t box_rows) {
+        return mn ? make_map_mn(map, base, is_bf16, p->k, p->n) : make_map(map, base, is_bf16, p->n, p->k, p->k, box_rows);
+    };
     for (uint32_t b = 0; b < p->batch; ++b) {
         const uint8_t *A = static_cast<const uint8_t *>(in[0]) + b * p->stride_a * es;
         const uint8_t *B = static_cast<const uint8_t *>(in[1]) + b * p->stride_b * es;
@@ -953,25 +997,26 @@ int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *c
             a.Y = Y, a.y_row_stride = p->n, a.y_col_stride = 1;
             a.C = C, a.c_row_stride = p->bias_row_stride, a.c_col_stride = p->bias_col_stride;
             if (bn == 256 && pl.splits == 1 && !pl.streamk_grid && p->m >= 512 && tc_pair_enabled()) {
-                if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !make_map(&mb, B, is_bf16, p->n, p->k, p->k, 128)) return RG_ERR_CUDA;
-                const int rc = is_bf16 ? tc_launch_pair<__nv_bfloat16>(ma, mb, a, st) : tc_launch_pair<__half>(ma, mb, a, st);
+                if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !map_b(&mb, B, 128)) return RG_ERR_CUDA;
+                const int rc = mn ? (is_bf16 ? tc_launch_pair<__nv_bfloat16, true>(ma, mb, a, st) : tc_launch_pair<__half, true>(ma, mb, a, st))
+                                  : (is_bf16 ? tc_launch_pair<__nv_bfloat16>(ma, mb, a, st) : tc_launch_pair<__half>(ma, mb, a, st));
                 if (rc != RG_OK) return rc;
                 continue;
             }
-            if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !make_map(&mb, B, is_bf16, p->n, p->k, p->k, bn)) return RG_ERR_CUDA;
+            if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !map_b(&mb, B, bn)) return RG_ERR_CUDA;
         } else {
             bn = p->m <= 32 ? 32 : 64;
             a.m = p->n, a.n = p->m;
             a.early = (p->flags & RG_MM_B_STATIC) ? 1u : 0u;
             a.Y = Y, a.y_row_stride = 1, a.y_col_stride = p->n;
             a.C = C, a.c_row_stride = p->bias_col_stride, a.c_col_stride = p->bias_row_stride;
-            if (!make_map(&ma, B, is_bf16, p->n, p->k, p->k, TC_BM) || !make_map(&mb, A, is_bf16, p->m, p->k, p->k, bn)) return RG_ERR_CUDA;
+            if (!map_b(&ma, B, TC_BM) || !make_map(&mb, A, is_bf16, p->m, p->k, p->k, bn)) return RG_ERR_CUDA;
         }
         int rc;
-#define RG_TC(T)                                                                        \
-    (bn == 256 ? tc_launch<T, 256, 4>(ma, mb, a, st) : bn == 128 ? tc_launch<T, 128, 6>(ma, mb, a, st) \
-     : bn == 64 ? tc_launch<T, 64, 8>(ma, mb, a, st) : tc_launch<T, 32, 8>(ma, mb, a, st))
-        rc = is_bf16 ? RG_TC(__nv_bfloat16) : RG_TC(__half);
+#define RG_TC(T, MN)                                                                                                           \
+    (bn == 256 ? tc_launch<T, 256, 4, false, MN>(ma, mb, a, st) : bn == 128 ? tc_launch<T, 128, 6, false, MN>(ma, mb, a, st) \
+     : bn == 64 ? tc_launch<T, 64, 8, false, MN>(ma, mb, a, st) : tc_launch<T, 32, 8, false, MN>(ma, mb, a, st))
+        rc = mn ? (is_bf16 ? RG_TC(__nv_bfloat16, true) : RG_TC(__half, true)) : (is_bf16 ? RG_TC(__nv_bfloat16, false) : RG_TC(__half, false));
 #undef RG_TC
         if (rc != RG_OK) return rc;
     }

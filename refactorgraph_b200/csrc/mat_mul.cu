@@ -55,7 +55,7 @@ extern "C" {
 
 size_t rg_b200_mat_mul_workspace(const rg_mat_mul_params *p) {
     // the tensor-core kernel's split-K path and the skinny kernel's k-split need scratch; sized for whichever could be chosen
-    if (!p || (p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a || !p->trans_b) return 0;
+    if (!p || (p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a) return 0;
     size_t bytes = gemm_tc_workspace(p);
     if (skinny_shape(p)) {
         const size_t s = linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0);

@@ -92,6 +92,17 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
     d |= static_cast<uint64_t>(2) << 61;
     return d;
 }
+// The same for an MN-major operand: rows of 128 bytes hold 64 consecutive m (or n), the next 64 are `block` bytes further
+// (leading byte offset), the next eight k-rows 1 KiB further (stride byte offset).
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t smem_addr, uint32_t block) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>((block >> 4) & 0x3FFFu) << 16;
+    d |= static_cast<uint64_t>(1024 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
 // Instruction descriptor for kind::f16: D fp32 (bits 4-5 = 1), A/B format (0 fp16, 1 bf16) at bits 7-9 / 10-12,
 // both operands K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
 __host__ __device__ inline uint32_t instr_desc(int is_bf16, uint32_t M, uint32_t N) {

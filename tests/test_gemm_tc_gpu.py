@@ -61,6 +61,27 @@ def test_pairs_of_ctas(dtype, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", HALF)
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 512), (4, 1032, 64), (7, 1000, 1032), (33, 22016, 512), (64, 128, 72), (65, 64, 64), (100, 304, 72),
+                                   (129, 136, 4096), (300, 4096, 1024), (511, 256, 200), (512, 264, 64), (700, 1000, 4096)])
+def test_weights_stored_k_by_n(dtype, m, n, k):
+    """trans_b = 0: the weights enter as an MN-major operand (on either side of the instruction, single CTAs and pairs).  Integer
+    data is exact in fp32 accumulation; the tolerance of the random data is the one of the K-major products."""
+    rng = np.random.default_rng(m + 3 * n + k)
+    a = rng.integers(-3, 4, (m, k)).astype(np.float32)
+    b = rng.integers(-1, 2, (k, n)).astype(np.float32)
+    yt = ops.mat_mul(ops.dev(a).to(dtype), ops.dev(b).to(dtype), force=3)
+    assert _ok()
+    assert torch.equal(yt.cpu(), torch.from_numpy(a @ b).to(dtype))
+    a = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(dtype)
+    b = torch.from_numpy((0.05 * rng.standard_normal((k, n))).astype(np.float32)).to(dtype)
+    c = torch.from_numpy(rng.standard_normal((m, n)).astype(np.float32)).to(dtype)
+    y2 = ops.mat_mul(a.cuda(), b.cuda(), c.cuda(), alpha=0.5, beta=2.0, force=3)
+    assert _ok()
+    want = onp.mat_mul(a.float().numpy(), b.float().numpy(), c.float().numpy(), alpha=0.5, beta=2.0)
+    np.testing.assert_allclose(y2.float().cpu().numpy(), want, atol=4e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("dtype", HALF)
 def test_pairs_of_ctas_bias_vector_and_batch(dtype):
     """The pair kernel behind the batched call with a broadcast bias row (element-wise loads of C)."""
     rng = np.random.default_rng(11)
