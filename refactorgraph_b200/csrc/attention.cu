@@ -8,8 +8,8 @@
 //    double-buffered shared-memory ring by cp.async.bulk (one copy per tile, or per 16-token page) completing on
 //    mbarriers; scores, online softmax and P*V run from shared memory with conflict-free 128-bit loads; the
 //    per-split (max, sum, acc) records go to the workspace and the last CTA to arrive merges them.
-//  * kv_append_kernel / attn_rows_kernel — cache append and a general (prefill or decode) kernel on the
-//    reference tensor layout, one warp per query row with online softmax.
+//  * kv_append_kernel — cache append of the reference-layout operator, whose attention itself runs in attn_prefill.cu (16-bit
+//    prompts at head_dim 128) or attn_rows.cu (everything else).
 #include "common.cuh"
 #include <cstdlib>
 
@@ -538,51 +538,6 @@ __global__ void kv_prefix_copy_kernel(const T *__restrict__ src, T *__restrict__
     }
 }
 
-// One warp per query row; lane owns EP = D/32 consecutive dims.  K/V rows are [.., kv_stride_tokens, D].
-template<class T, int EP>
-__global__ void __launch_bounds__(128) attn_rows_kernel(const T *__restrict__ q, const T *__restrict__ K,
-                                                        const T *__restrict__ V, T *__restrict__ o,
-                                                        const int64_t *__restrict__ past_p, uint32_t batch,
-                                                        uint32_t n_heads, uint32_t n_kv, uint32_t S,
-                                                        uint32_t kv_tokens /* tokens per (n, kv head) in K/V */,
-                                                        float scale) {
-    constexpr int D = EP * 32;
-    const uint32_t past = past_clamped(past_p, kv_tokens);
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t row = static_cast<uint64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);// (n, h, i)
-    if (row >= static_cast<uint64_t>(batch) * n_heads * S) return;
-    const uint32_t i = static_cast<uint32_t>(row % S);
-    const uint32_t h = static_cast<uint32_t>((row / S) % n_heads);
-    const uint32_t n = static_cast<uint32_t>(row / S / n_heads);
-    const uint32_t kvh = h / (n_heads / n_kv);
-    const T *Kb = K + (static_cast<size_t>(n) * n_kv + kvh) * kv_tokens * D;
-    const T *Vb = V + (static_cast<size_t>(n) * n_kv + kvh) * kv_tokens * D;
-    float qv[EP], acc[EP];
-#pragma unroll
-    for (int e = 0; e < EP; ++e) {
-        qv[e] = Num<T>::to_f(q[row * D + lane * EP + e]) * scale;
-        acc[e] = 0.f;
-    }
-    float m = -INFINITY, l = 0.f;
-    const uint32_t last = past + i;// keys 0..last inclusive
-    for (uint32_t j = 0; j <= last && j < kv_tokens; ++j) {
-        float dot = 0.f;
-#pragma unroll
-        for (int e = 0; e < EP; ++e) dot += qv[e] * Num<T>::to_f(Kb[static_cast<size_t>(j) * D + lane * EP + e]);
-        dot = warp_sum(dot);
-        const float mn = fmaxf(m, dot);
-        const float corr = m == -INFINITY ? 0.f : expf(m - mn);
-        const float p = expf(dot - mn);
-        l = l * corr + p;
-#pragma unroll
-        for (int e = 0; e < EP; ++e)
-            acc[e] = acc[e] * corr + p * Num<T>::to_f(Vb[static_cast<size_t>(j) * D + lane * EP + e]);
-        m = mn;
-    }
-#pragma unroll
-    for (int e = 0; e < EP; ++e) o[row * D + lane * EP + e] = Num<T>::from_f(acc[e] / l);
-}
-
 // grouped-query variant (attn_decode_gqa.cu): one CTA serves all query heads of a KV head
 bool attn_decode_gqa_applies(const rg_attn_decode_params *p);
 size_t attn_decode_gqa_workspace(const rg_attn_decode_params *p);
@@ -592,8 +547,12 @@ int attn_decode_gqa_launch(const rg_attn_decode_params *p, void *ws, const void 
 int attn_prefill_ref_layout(int dtype, const void *q, const void *K, const void *V, void *o, const int64_t *past, uint32_t batch,
                             uint32_t n_heads, uint32_t n_kv, uint32_t S, uint32_t kv_tokens, cudaStream_t st);
 
+// fp32-probability kernel on the reference layout (attn_rows.cu)
+size_t attn_rows_workspace(const rg_attention_params *p);
+int attn_rows(const rg_attention_params *p, void *ws, const void *q, const void *k, const void *v, void *o, const int64_t *past, uint32_t kv_tokens, cudaStream_t st);
+
 template<class T>
-static int attention_launch(const rg_attention_params *p, const void *const *in, void *const *out, cudaStream_t st) {
+static int attention_launch(const rg_attention_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
     auto q = static_cast<const T *>(in[0]);
     auto k = static_cast<const T *>(in[1]);
     auto v = static_cast<const T *>(in[2]);
@@ -628,19 +587,7 @@ static int attention_launch(const rg_attention_params *p, const void *const *in,
     // tensor-core flash kernel for 16-bit types at head_dim 128 once there is a tile's worth of query rows
     if (sizeof(T) == 2 && p->head_dim == 128 && p->seq_len >= 16 && aligned16(q) && aligned16(K) && aligned16(V) && aligned16(o))
         return attn_prefill_ref_layout(p->dtype, q, K, V, o, past, p->batch, p->n_heads, p->n_kv_heads, p->seq_len, kv_tokens, st);
-    const unsigned grid = static_cast<unsigned>((rows + 3) / 4);
-    const float scale = 1.0f / sqrtf(static_cast<float>(p->head_dim));
-#define RG_ATT(EP) attn_rows_kernel<T, EP><<<grid, 128, 0, st>>>(q, K, V, o, past, p->batch, p->n_heads, p->n_kv_heads, p->seq_len, kv_tokens, scale)
-    switch (p->head_dim) {
-        case 32: RG_ATT(1); break;
-        case 64: RG_ATT(2); break;
-        case 128: RG_ATT(4); break;
-        case 256: RG_ATT(8); break;
-        default: return RG_ERR_SHAPE;
-    }
-#undef RG_ATT
-    count_launch();
-    return launch_status();
+    return attn_rows(p, ws, q, K, V, o, past, kv_tokens, st);
 }
 
 int attn_error_word(bool clear) { return error_symbol(s_attn_error, clear); }
@@ -661,16 +608,19 @@ static bool attn_pdl_enabled() {
 
 extern "C" {
 
-size_t rg_b200_attention_workspace(const rg_attention_params *) { return 0; }
-int rg_b200_attention(const rg_attention_params *p, void *, const void *const *in, void *const *out, void *stream) {
+size_t rg_b200_attention_workspace(const rg_attention_params *p) {
+    if (!p || p->n_kv_heads == 0 || p->n_heads % p->n_kv_heads != 0) return 0;
+    return attn_rows_workspace(p);
+}
+int rg_b200_attention(const rg_attention_params *p, void *ws, const void *const *in, void *const *out, void *stream) {
     if (!p || !in || !out || !in[0] || !in[1] || !in[2] || !out[0]) return RG_ERR_NULL;
     if (p->n_kv_heads == 0 || p->n_heads % p->n_kv_heads != 0) return RG_ERR_SHAPE;
     if (p->has_cache && p->max_seq < p->seq_len) return RG_ERR_SHAPE;
     auto st = static_cast<cudaStream_t>(stream);
     switch (p->dtype) {
-        case RG_F32: return attention_launch<float>(p, in, out, st);
-        case RG_FP16: return attention_launch<__half>(p, in, out, st);
-        case RG_BF16: return attention_launch<__nv_bfloat16>(p, in, out, st);
+        case RG_F32: return attention_launch<float>(p, ws, in, out, st);
+        case RG_FP16: return attention_launch<__half>(p, ws, in, out, st);
+        case RG_BF16: return attention_launch<__nv_bfloat16>(p, ws, in, out, st);
         default: return RG_ERR_DTYPE;
     }
 }

@@ -262,8 +262,11 @@ def attention(q, k, v, past=None, k_cache=None, v_cache=None):
     has_cache = k_cache is not None
     p = capi.AttentionParams(DT[q.dtype], N, nH, k.shape[1], S, D, k_cache.shape[2] if has_cache else S, int(has_cache))
     pt = None if past is None else torch.tensor([past], dtype=torch.int64, device=q.device)
+    nws = capi.workspace("attention", p)
+    ws = torch.zeros(max(nws, 1), dtype=torch.uint8, device=q.device)
     capi.call("attention", p, [ptr(q), ptr(k), ptr(v), ptr(pt), ptr(k_cache), ptr(v_cache)],
-              [ptr(o), ptr(k_cache), ptr(v_cache)], stream=stream())
+              [ptr(o), ptr(k_cache), ptr(v_cache)], ws=ptr(ws) if nws else 0, stream=stream())
+    torch.cuda.current_stream().synchronize()  # the workspace is released on return
     return o
 
 
