@@ -22,6 +22,10 @@ size_t gemm_tc_workspace(const rg_mat_mul_params *p);// split-K partials + arriv
 // rank's all-reduce slots on the peers instead of into Y (in = {A, B}); RG_ERR_UNSUPPORTED for any other shape
 int gemm_tc_push(const rg_mat_mul_params *p, void *ws, const void *const *in, const ArPeers &peers, cudaStream_t st);
 bool gemm_tc_supported(const rg_mat_mul_params *p, const void *const *in, void *const *out);
+// fp32 product on the tensor cores, three bf16 parts per operand (gemm_tc32.cu); trans_a = 0
+bool gemm_tc32_preferred(const rg_mat_mul_params *p);
+size_t gemm_tc32_workspace(const rg_mat_mul_params *p);// split-K partials and arrival counters (zero before first use)
+int gemm_tc32(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st);
 // Weight-streaming linear layer for 5..32 rows of X on the warp-level tensor path (linear_skinny.cu).
 struct SkinnyCall {
     int dtype;
@@ -43,6 +47,7 @@ int linear_skinny(const SkinnyCall &c, void *ws, const void *const *in, void *co
 int linear_error_word(bool clear);
 int attn_error_word(bool clear);
 int gemm_tc_error_word(bool clear);
+int gemm_tc32_error_word(bool clear);
 int all_reduce_error_word(bool clear);
 int mega_error_word(bool clear);
 int linear_index_error_word(bool clear);

@@ -55,7 +55,9 @@ extern "C" {
 
 size_t rg_b200_mat_mul_workspace(const rg_mat_mul_params *p) {
     // the tensor-core kernel's split-K path and the skinny kernel's k-split need scratch; sized for whichever could be chosen
-    if (!p || (p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a) return 0;
+    if (!p || p->m == 0 || p->n == 0 || p->k == 0 || p->batch == 0) return 0;
+    if (p->dtype == RG_F32) return gemm_tc32_preferred(p) || (p->force_kernel == 5 && !p->trans_a) ? gemm_tc32_workspace(p) : 0;
+    if ((p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a) return 0;
     size_t bytes = gemm_tc_workspace(p);
     if (skinny_shape(p)) {
         const size_t s = linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0);
@@ -78,8 +80,10 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         case 2: return gemv_shape(p) ? run_gemv(p, in, out, st) : RG_ERR_UNSUPPORTED;
         case 3: return gemm_tc_supported(p, in, out) ? gemm_tc(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
         case 4: return skinny_shape(p) ? run_skinny(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
+        case 5: return gemm_tc32(p, ws, in, out, st);
         default: return RG_ERR_UNSUPPORTED;
     }
+    if (p->dtype == RG_F32) return gemm_tc32_preferred(p) ? gemm_tc32(p, ws, in, out, st) : gemm_simt(p, in, out, st);
     if (gemv_shape(p) && aligned16(in[0]) && aligned16(in[1])) {
         const int rc = run_gemv(p, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;
