@@ -600,3 +600,21 @@ def test_no_bounded_wait_expired():
     torch.cuda.synchronize()
     assert capi.load().rg_b200_launch_count() > 0
     assert capi.load().rg_b200_error_state() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32] + HALF)
+@pytest.mark.parametrize("rows,n,k", [(1, 1024, 1), (3, 4096, 64), (2, 4104, 7), (2, 16384, 50), (1, 32768, 5), (2, 65536, 3), (150, 1031, 2)])
+def test_topk_rows_in_registers(rows, n, k, dtype):
+    """Row lengths on both sides of every register form; rows whose repeated values push them to the radix select; NaNs; an offset base."""
+    rng = np.random.default_rng(n + k)
+    x = rnd16(rng.standard_normal((rows, n)).astype(np.float32), dtype)
+    x[0, ::3] = 2.0                      # more than 512 of them at or above the threshold
+    x[-1, 5], x[-1, 17] = np.nan, np.inf
+    if rows > 1:
+        x[1, :] = np.nan                 # fewer than k numbers in the row
+        x[1, 9] = -1.0
+    for xd in (ops.dev(x, dtype), torch.cat([torch.zeros(1, dtype=dtype, device="cuda"), ops.dev(x, dtype).flatten()])[1:].view(rows, n)):
+        vals, idx = ops.topk(xd, k)
+        wv, wi = onp.topk(x, k)
+        np.testing.assert_array_equal(idx.cpu().numpy(), wi)
+        np.testing.assert_array_equal(vals.float().cpu().numpy(), wv)
