@@ -506,20 +506,20 @@ static int decode_launch(const rg_attn_decode_params *p, void *ws, const void *c
 }
 
 // ---- reference-layout kernels -----------------------------------------------------------------------
-// cache[n, h, past + s, :] = x[n, h, s, :]
-template<class T>
-__global__ void kv_append_kernel(const T *__restrict__ k, const T *__restrict__ v, T *__restrict__ kc,
-                                 T *__restrict__ vc, const int64_t *__restrict__ past_p, uint32_t nh, uint32_t S,
-                                 uint32_t D, uint32_t max_seq, uint64_t total) {
+// cache[n, h, past + s, :] = x[n, h, s, :] in units of U (16 bytes where everything is aligned to them), `row` units per token
+template<class U>
+__global__ void kv_append_kernel(const U *__restrict__ k, const U *__restrict__ v, U *__restrict__ kc, U *__restrict__ vc,
+                                 const int64_t *__restrict__ past_p, uint32_t S, uint32_t row, uint32_t max_seq, uint64_t total) {
+    pdl_enter();
     const uint32_t past = past_clamped(past_p, max_seq);
     for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
          t += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint32_t d = static_cast<uint32_t>(t % D);
-        const uint64_t r = t / D;
-        const uint32_t s = static_cast<uint32_t>(r % S);
-        const uint64_t nhh = r / S;// n*nh + h
+        const uint64_t r = t / row;
+        const uint32_t d = static_cast<uint32_t>(t - r * row);
+        const uint64_t nhh = r / S;// n * KV heads + KV head
+        const uint32_t s = static_cast<uint32_t>(r - nhh * S);
         if (past + s >= max_seq) continue;
-        const uint64_t dst = (nhh * max_seq + past + s) * D + d;
+        const uint64_t dst = (nhh * max_seq + past + s) * row + d;
         kc[dst] = k[t];
         vc[dst] = v[t];
     }
@@ -575,9 +575,15 @@ static int attention_launch(const rg_attention_params *p, void *ws, const void *
         }
         const uint64_t total = heads * p->seq_len * p->head_dim;
         if (total) {
-            const uint64_t want = (total + 255) / 256;
-            kv_append_kernel<T><<<static_cast<unsigned>(want > cap ? cap : want), 256, 0, st>>>(
-                k, v, kco, vco, past, p->n_kv_heads, p->seq_len, p->head_dim, p->max_seq, total);
+            constexpr uint32_t N = 16 / sizeof(T);
+            const bool wide = p->head_dim % N == 0 && aligned16(k) && aligned16(v) && aligned16(kco) && aligned16(vco);
+            const uint64_t units = wide ? total / N : total, want = (units + 255) / 256;
+            const dim3 grid(static_cast<unsigned>(want > cap ? cap : want));
+            if (wide)
+                RG_CHECK_CUDA(launch_pdl(kv_append_kernel<uint4>, grid, dim3(256), 0, st, reinterpret_cast<const uint4 *>(k), reinterpret_cast<const uint4 *>(v),
+                                         reinterpret_cast<uint4 *>(kco), reinterpret_cast<uint4 *>(vco), past, p->seq_len, p->head_dim / N, p->max_seq, units));
+            else
+                RG_CHECK_CUDA(launch_pdl(kv_append_kernel<T>, grid, dim3(256), 0, st, k, v, kco, vco, past, p->seq_len, p->head_dim, p->max_seq, units));
             count_launch();
         }
         K = kco, V = vco, kv_tokens = p->max_seq;

@@ -202,13 +202,14 @@ __global__ void softmax_row_kernel(const T *__restrict__ x, T *__restrict__ y, u
     }
 }
 
-// post == 1, rows of up to 8192 16-byte chunks: the row lives in registers (CH chunks per thread), so it is read once and
+// post == 1, rows of up to 8192 16-byte chunks (VEC) or single elements: the row lives in registers (CH chunks per thread), so it is read once and
 // every element costs one exponential: maximum, then exp and sum, then the scaled store.  (The online kernel above pays two
 // exponentials per element and reads the row twice: on [65536, 2048] fp16 it measured 289 us, issue-bound at 93 % SM throughput.)
-template<class T, int CH>
+template<class T, int CH, bool VEC>
 __global__ void __launch_bounds__(1024) softmax_row_reg_kernel(const T *__restrict__ x, T *__restrict__ y, uint32_t n) {
-    constexpr int N = Vec16<T>::N;
+    constexpr int N = VEC ? Vec16<T>::N : 1;
     __shared__ float red[33];
+    pdl_enter();
     const uint32_t chunks = n / N;
     const T *xr = x + static_cast<size_t>(blockIdx.x) * n;
     T *yr = y + static_cast<size_t>(blockIdx.x) * n;
@@ -218,9 +219,13 @@ __global__ void __launch_bounds__(1024) softmax_row_reg_kernel(const T *__restri
     for (int i = 0; i < CH; ++i) {
         const uint32_t c = threadIdx.x + i * blockDim.x;
         if (c < chunks) {
-            Vec16<T> a;
-            a.load(xr + c * N);
-            a.unpack(v[i]);
+            if constexpr (VEC) {
+                Vec16<T> a;
+                a.load(xr + c * N);
+                a.unpack(v[i]);
+            } else {
+                v[i][0] = Num<T>::to_f(xr[c]);
+            }
 #pragma unroll
             for (int j = 0; j < N; ++j) m = fmaxf(m, v[i][j]);
         }
@@ -246,9 +251,13 @@ __global__ void __launch_bounds__(1024) softmax_row_reg_kernel(const T *__restri
         if (c < chunks) {
 #pragma unroll
             for (int j = 0; j < N; ++j) v[i][j] *= inv;
-            Vec16<T> a;
-            a.pack(v[i]);
-            a.store(yr + c * N);
+            if constexpr (VEC) {
+                Vec16<T> a;
+                a.pack(v[i]);
+                a.store(yr + c * N);
+            } else {
+                yr[c] = Num<T>::from_f(v[i][0]);
+            }
         }
     }
 }
@@ -279,17 +288,21 @@ static int softmax_launch(const rg_softmax_params *p, const void *const *in, voi
         const uint32_t work = vec ? p->mid / N : p->mid;
         uint32_t threads = work >= 2048 ? 1024 : work >= 256 ? 256 : (work + 31) / 32 * 32;
         if (threads < 32) threads = 32;
-        if (vec && work <= 8192) {
+        if (work <= 8192) {
             uint32_t ch = (work + 1023) / 1024;
             ch = ch <= 1 ? 1 : ch <= 2 ? 2 : ch <= 4 ? 4 : 8;
             uint32_t t = ((work + ch - 1) / ch + 31) / 32 * 32;
             if (t < 32) t = 32;
+#define RG_SOFTMAX(CH) \
+    RG_CHECK_CUDA(vec ? launch_pdl(softmax_row_reg_kernel<T, CH, true>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid) \
+                      : launch_pdl(softmax_row_reg_kernel<T, CH, false>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid))
             switch (ch) {
-                case 1: softmax_row_reg_kernel<T, 1><<<p->pre, t, 0, st>>>(x, y, p->mid); break;
-                case 2: softmax_row_reg_kernel<T, 2><<<p->pre, t, 0, st>>>(x, y, p->mid); break;
-                case 4: softmax_row_reg_kernel<T, 4><<<p->pre, t, 0, st>>>(x, y, p->mid); break;
-                default: softmax_row_reg_kernel<T, 8><<<p->pre, t, 0, st>>>(x, y, p->mid); break;
+                case 1: RG_SOFTMAX(1); break;
+                case 2: RG_SOFTMAX(2); break;
+                case 4: RG_SOFTMAX(4); break;
+                default: RG_SOFTMAX(8); break;
             }
+#undef RG_SOFTMAX
         } else if (vec) softmax_row_kernel<T, true><<<p->pre, threads, 0, st>>>(x, y, p->mid);
         else
             softmax_row_kernel<T, false><<<p->pre, threads, 0, st>>>(x, y, p->mid);

@@ -618,3 +618,35 @@ def test_topk_rows_in_registers(rows, n, k, dtype):
         wv, wi = onp.topk(x, k)
         np.testing.assert_array_equal(idx.cpu().numpy(), wi)
         np.testing.assert_array_equal(vals.float().cpu().numpy(), wv)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.uint8, torch.float64])
+@pytest.mark.parametrize("shape,perm", [((7, 33, 65), (0, 2, 1)), ((2, 16, 31, 17), (0, 1, 3, 2)), ((3, 40, 2, 50), (3, 2, 1, 0)), ((1, 509, 4, 64), (0, 2, 1, 3)),
+                                        ((5, 6, 24), (1, 0, 2)), ((33, 1), (1, 0)), ((100, 200), (1, 0)), ((4, 3, 2, 15), (2, 0, 1, 3))])
+def test_transpose_tiles_and_wide_runs(shape, perm, dtype):
+    x = (torch.arange(int(np.prod(shape))) % 251).reshape(shape).to(dtype).cuda()
+    p = capi.TransposeParams()
+    p.rank, p.elem_bytes = len(shape), x.element_size()
+    for d in range(len(shape)):
+        p.in_shape[d], p.perm[d] = shape[d], perm[d]
+    for off in (0, 1):  # a base on and off a 16-byte boundary
+        src = torch.cat([torch.zeros(off, dtype=dtype, device="cuda"), x.flatten()])[off:]
+        y = torch.empty([shape[i] for i in perm], dtype=dtype, device="cuda")
+        capi.call("transpose", p, [src.data_ptr()], [y.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(y, x.permute(*perm).contiguous())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32] + HALF)
+def test_binary_with_one_value_and_softmax_of_odd_rows(dtype):
+    rng = np.random.default_rng(3)
+    x = rnd16(rng.standard_normal((3, 5, 8)).astype(np.float32), dtype)
+    s = rnd16(np.float32([1.7]), dtype)
+    for op, f in ((3, np.divide), (1, np.subtract)):
+        y = ops.binary(op, ops.dev(x, dtype), ops.dev(s, dtype))
+        want = torch.from_numpy(f(x, s).astype(np.float32)).to(dtype).float().numpy()
+        np.testing.assert_allclose(y.float().cpu().numpy(), want, rtol=2e-7 if dtype == torch.float32 else 1e-2)
+    for n in (1, 31, 509, 1025, 4097, 8193):
+        x = rnd16((3 * rng.standard_normal((4, n))).astype(np.float32), dtype)
+        x[1, n // 2] = -np.inf if n > 1 else 0.0
+        y = ops.softmax(ops.dev(x, dtype), 1)
+        np.testing.assert_allclose(y.float().cpu().numpy(), onp.softmax_intended(x, 1), rtol=2e-5 if dtype == torch.float32 else 1e-2, atol=1e-9 if dtype == torch.float32 else 2e-3)
