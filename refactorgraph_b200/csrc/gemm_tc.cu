@@ -533,6 +533,11 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                         // this thread's row of every split: the BN/4 loads of one split are independent, so the sum
                         // costs one L2 round trip per split (fixed split order => deterministic)
                         float4 acc[BN / 4];
+                        float add[BN];// this row of C: all loads in flight beside those of the sums (behind the stores of Y, which may
+                                      // be the same memory as far as the compiler knows, each would wait for its own round trip)
+#pragma unroll
+                        for (int c = 0; c < BN; ++c)
+                            add[c] = C && n0 + c < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(n0 + c) * a.c_col_stride]) : 0.f;
 #pragma unroll
                         for (int c = 0; c < BN / 4; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
@@ -552,7 +557,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                                 const uint32_t col = n0 + c * 4 + j;
                                 if (col < a.n) {
                                     float v = a.alpha * vals[j];
-                                    if (C) v += a.beta * Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]);
+                                    if (C) v += a.beta * add[c * 4 + j];
                                     Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(col) * a.y_col_stride] = Num<T>::from_f(v);
                                 }
                             }
@@ -712,26 +717,40 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     continue;
                 }
             }
+            // 32 columns at a time.  What is added from C is fetched ahead of the accumulator (behind the stores of the columns before,
+            // which may be the same memory as far as the compiler knows, every load would wait for its own round trip): one residual
+            // tile of 128 x 256 took 12 us longer than the plain product with a load in front of every store.
+            const bool rows_wide = a.y_col_stride == 1 && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor);
+            Vec16<T> cnext[4];
+            auto fetch_c = [&](int c0) {
+                if (C && rows_wide && row < a.m && n0 + c0 + 32 <= a.n) {
+                    const T *csrc = C + static_cast<uint64_t>(row) * a.c_row_stride + n0 + c0;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) cnext[j].load(csrc + 8 * j);
+                }
+            };
+            fetch_c(0);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t r[32];
+                Vec16<T> cv[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cv[j] = cnext[j];
+                if (c0 + 32 < BN) fetch_c(c0 + 32);
                 tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
                 tmem_ld_wait();
                 if (row < a.m) {
-                    if (a.y_col_stride == 1 && n0 + c0 + 32 <= a.n && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor)) {
-                        // contiguous 64-byte run of this thread's row: four 16-byte stores (and loads of C)
+                    if (rows_wide && n0 + c0 + 32 <= a.n) {
+                        // contiguous 64-byte run of this thread's row: four 16-byte stores
                         T *dst = Y + static_cast<uint64_t>(row) * a.y_row_stride + n0 + c0;
-                        const T *csrc = C ? C + static_cast<uint64_t>(row) * a.c_row_stride + n0 + c0 : nullptr;
 #pragma unroll
                         for (int j = 0; j < 32; j += 8) {
                             float f[8];
 #pragma unroll
                             for (int e = 0; e < 8; ++e) f[e] = a.alpha * __uint_as_float(r[j + e]);
-                            if (csrc) {
-                                Vec16<T> cv;
+                            if (C) {
                                 float cf[8];
-                                cv.load(csrc + j);
-                                cv.unpack(cf);
+                                cv[j / 8].unpack(cf);
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) f[e] += a.beta * cf[e];
                             }
@@ -740,12 +759,18 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                             v.store(dst + j);
                         }
                     } else {
+                        float add[32];
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const uint32_t col = n0 + c0 + j;
+                            add[j] = C && col < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]) : 0.f;
+                        }
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const uint32_t col = n0 + c0 + j;
                             if (col < a.n) {
                                 float v = a.alpha * __uint_as_float(r[j]);
-                                if (C) v += a.beta * Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]);
+                                if (C) v += a.beta * add[j];
                                 Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(col) * a.y_col_stride] = Num<T>::from_f(v);
                             }
                         }
