@@ -6,21 +6,18 @@ struct ArPeers;
 int gemm_simt(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st);
 int linear_stream(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
 // tcgen05/TMEM GEMM: Y[m,n] = alpha * A[m,k] * B[n,k]^T (+ beta*C), fp16/bf16, fp32 accumulation in TMEM.
-int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st);
+int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st);
 int gemm_tc_swiglu(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
-// SiLU gate on 5..64 tokens: weights on the instruction's M side, k-split plan of the skinny product (workspace as reported)
+// SiLU gate on 5..64 tokens: weights on the instruction's M side, k split as for the skinny product
 bool gemm_tc_swiglu_small_shape(const rg_linear_params *p);
-size_t gemm_tc_swiglu_small_workspace(const rg_linear_params *p);
-int gemm_tc_swiglu_small(const rg_linear_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st);
+int gemm_tc_swiglu_small(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
 // QKV split + RoPE + cache append on 5..64 tokens, same orientation (a 128-row tile = one head of head_dim 128)
 bool gemm_tc_qkv_rope_small_shape(const rg_linear_params *p);
-size_t gemm_tc_qkv_rope_small_workspace(const rg_linear_params *p);
-int gemm_tc_qkv_rope_small(const rg_linear_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st);
+int gemm_tc_qkv_rope_small(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
 int gemm_tc_qkv_rope(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
-size_t gemm_tc_workspace(const rg_mat_mul_params *p);// split-K partials + arrival counters (zero before first use)
 // The product of up to 64 tokens whose 16-bit result goes, paired with the flag of the communicator's call in flight, into this
 // rank's all-reduce slots on the peers instead of into Y (in = {A, B}); RG_ERR_UNSUPPORTED for any other shape
-int gemm_tc_push(const rg_mat_mul_params *p, void *ws, const void *const *in, const ArPeers &peers, cudaStream_t st);
+int gemm_tc_push(const rg_mat_mul_params *p, const void *const *in, const ArPeers &peers, cudaStream_t st);
 bool gemm_tc_supported(const rg_mat_mul_params *p, const void *const *in, void *const *out);
 // fp32 product on the tensor cores, three bf16 parts per operand (gemm_tc32.cu); trans_a = 0
 bool gemm_tc32_preferred(const rg_mat_mul_params *p);

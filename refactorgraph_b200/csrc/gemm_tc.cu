@@ -30,6 +30,7 @@ static __device__ int s_tc_index_error;// a cache-append position or block-table
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;// 64 x 2 B = one 128-byte swizzle row
 constexpr int TC_THREADS = 192;
+__host__ __device__ constexpr uint32_t tc_recv_bytes(int bn) { return bn <= 64 ? 128u * bn * 4u : 0u; }// a tile's sums, from all CTAs of a cluster
 constexpr uint32_t TC_MN_BLOCK = 64 * TC_BK * 2;// one box of an MN-major operand: 64 columns x 64 k-rows
 
 struct TcArgs {
@@ -40,10 +41,7 @@ struct TcArgs {
     uint32_t c_row_stride, c_col_stride;
     uint64_t y_row_stride, y_col_stride;// element strides of Y over the kernel's (row, col) = lets swapped runs write Y^T
     int is_bf16;
-    uint32_t splits;   // partial slots per output tile: the k-splits (1 = none), or with streamk the most CTAs a tile can span
-    uint32_t streamk;  // != 0: CTA c owns the contiguous run [U c / G, U (c+1) / G) of the U = tiles * kblocks (tile, k-block) units
-    float *partial;    // [tiles][splits][128][BN] fp32, used when splits > 1
-    unsigned *counter; // [tiles] arrival counters, zero before the first call and left at zero
+    uint32_t ksplit;   // CTAs of a cluster that share a tile, each with its part of k (skinny forms; 1 elsewhere)
     uint32_t group_m;  // row tiles per group of the tile order
     uint32_t early;    // operand that no earlier kernel of the stream writes (a weight): 1 = A, 2 = B, 0 = neither
     // QKV epilogue (rope != 0): columns are [q heads | k heads | v heads] of head_dim 128, rows are tokens; q is rotated into
@@ -96,45 +94,18 @@ __device__ __forceinline__ void tile_coords(uint32_t t, uint32_t m_tiles, uint32
     nt = r / rows;
 }
 
-// One CTA's work, as (tile, k-block range) segments.  Split mode: items c, c + G, ... of tiles * splits, item = (tile, split).
-// Stream-K mode: a contiguous run of (tile, k-block) units, so every CTA streams the same number of bytes whatever the tile
-// count; a tile that spans several CTAs is summed by the last of them to arrive (ord = this CTA's place among them).
-struct TcSeg {
-    uint32_t tile, kb0, kb1, ord, ncontrib;
-};
+// A unit's work: tiles unit, unit + units, ... over the k-blocks [kb0, kb1).  A unit is a CTA, a pair of CTAs (pair mode) or a cluster
+// of ksplit CTAs that divide the k-blocks of each tile between them.
 struct TcWalk {
-    uint32_t streamk, splits, kblocks, items, item, G;
-    uint64_t U, u, u1;
-    // unit = what walks the tiles: a CTA, or a pair of CTAs (pair mode: unit index and count are halved)
-    __device__ __forceinline__ void init(const TcArgs &a, uint32_t tiles, uint32_t kblocks_, uint32_t unit = blockIdx.x, uint32_t units = gridDim.x) {
-        streamk = a.streamk, splits = a.splits, kblocks = kblocks_, G = units;
-        items = tiles * a.splits, item = unit;
-        U = static_cast<uint64_t>(tiles) * kblocks_;
-        u = U * unit / G, u1 = U * (unit + 1) / G;
+    uint32_t tiles, units, item, kb0, kb1, tile;
+    __device__ __forceinline__ void init(uint32_t tiles_, uint32_t kblocks, uint32_t unit, uint32_t units_, uint32_t part, uint32_t parts) {
+        tiles = tiles_, units = units_, item = unit;
+        kb0 = kblocks * part / parts, kb1 = kblocks * (part + 1) / parts;
     }
-    // CTA that owns unit x: the largest c with floor(U c / G) <= x
-    __device__ __forceinline__ uint32_t owner(uint64_t x) const { return static_cast<uint32_t>(((x + 1) * G + U - 1) / U - 1); }
-    __device__ __forceinline__ bool next(TcSeg &s) {
-        if (!streamk) {
-            if (item >= items) return false;
-            const uint32_t ks = item % splits;
-            s.tile = item / splits, s.kb0 = kblocks * ks / splits, s.kb1 = kblocks * (ks + 1) / splits;
-            s.ord = ks, s.ncontrib = splits;
-            item += G;
-            return true;
-        }
-        if (u >= u1) return false;
-        s.tile = static_cast<uint32_t>(u / kblocks), s.kb0 = static_cast<uint32_t>(u % kblocks);
-        const uint64_t left = u1 - u;
-        s.kb1 = left < kblocks - s.kb0 ? s.kb0 + static_cast<uint32_t>(left) : kblocks;
-        u += s.kb1 - s.kb0;
-        if (s.kb0 == 0 && s.kb1 == kblocks) {
-            s.ord = 0, s.ncontrib = 1;
-        } else {
-            const uint64_t x0 = static_cast<uint64_t>(s.tile) * kblocks;
-            const uint32_t cf = owner(x0), cl = owner(x0 + kblocks - 1);
-            s.ord = blockIdx.x - cf, s.ncontrib = cl - cf + 1;
-        }
+    __device__ __forceinline__ bool next() {
+        if (item >= tiles) return false;
+        tile = item;
+        item += units;
         return true;
     }
 };
@@ -146,6 +117,14 @@ struct TcWalk {
 // the accumulator and its epilogue warps store them.  Per SM and k-block that is 32 KiB from L2 instead of 48 for the same 128 x 256
 // outputs: the single-CTA kernel is bound by requests to L2 (ncu: 68 % of request cycles, tensor pipe 80 %; an extra L2 prefetch
 // per box made it 22 % slower).  No load is multicast.
+//
+// k-split (skinny forms): a 128-row tile per CTA leaves most SMs idle or the last round nearly empty, so a cluster of 2, 4 or 8 CTAs
+// shares each tile, every CTA streaming its part of k.  CTA r finishes columns (tokens) [r W, r W + W), W = BN / ksplit: the others
+// store their sums of those columns into its receive buffer over distributed shared memory (st.shared::cluster, counted on its
+// recv_full mbarrier; recv_free, counted on the senders', hands the buffer back), it adds them in rank order and runs the
+// epilogue of its W columns.  Two receive buffers, so the exchange of a tile overlaps the stream of the next.
+// Measured with stream-K / parked partial sums in global memory before: 8 tokens x 4096 x 4096 16.4 -> 11.6 us, 4096 x 11008 24.9 ->
+// 19.8, 12288 x 4096 26.6 -> 23.2, 22016 x 4096 37.7 -> 36.5, 32000 x 4096 49.4 -> 47.1; an 8-layer 7B step of 8 sequences 1.37 -> 1.17 ms.
 //
 // MN: the weight matrix is stored [k, out] (MatMul with transB = 0, as exporters write it): its tile is loaded as boxes of 64 output
 // columns x 64 k-rows, one 8 KiB block per 64 columns, and enters the instruction as an MN-major operand (the M side of the skinny
@@ -159,15 +138,20 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     constexpr uint32_t ROWS = PAIR ? 2 * TC_BM : TC_BM;// rows of a tile
     constexpr bool MN_A = MN && BN <= 64, MN_B = MN && BN > 64;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;// 0 = the CTA that issues the products
-    const uint32_t unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const uint32_t S = PAIR || BN > 64 ? 1u : a.ksplit, part = S > 1 ? cluster_ctarank() : 0u;
+    const uint32_t unit = PAIR ? blockIdx.x >> 1 : blockIdx.x / S, units = PAIR ? gridDim.x >> 1 : gridDim.x / S;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // the swizzled tiles need 1024-byte alignment
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
+    uint8_t *recv = smem + STAGES * STAGE_BYTES;// [2][sender][4-column group][128 rows][4] fp32
+    constexpr uint32_t RECV_BYTES = tc_recv_bytes(BN);
+    uint64_t *full = reinterpret_cast<uint64_t *>(recv + 2 * RECV_BYTES);
     uint64_t *empty = full + STAGES;
     uint64_t *acc_full = empty + STAGES; // [2]
     uint64_t *acc_empty = acc_full + 2;  // [2]
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+    uint64_t *recv_full = acc_empty + 2; // [2]
+    uint64_t *recv_free = recv_full + 2; // [2]
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(recv_free + 2);
     int *failed = reinterpret_cast<int *>(tmem_slot + 1);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,6 +166,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], PAIR ? 8 : 4);// one arrival per epilogue warp (pair mode: of both CTAs, on the even CTA's barrier)
+            mbar_init(&recv_full[b], 4 * S);       // one per epilogue warp of every CTA of the cluster
+            mbar_init(&recv_free[b], 4 * S);
         }
         *failed = 0;
         fence_mbar_init();
@@ -198,6 +184,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) cluster_sync();// the partner's barriers are initialised before anything arrives on them
+    if (S > 1) cluster_arrive();       // the same; waited for where the first arrival is made
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Programmatic dependent launch: everything up to here, and the first stages of a weight operand, overlap the previous
@@ -233,15 +220,14 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 }
             };
             TcWalk walk;
-            walk.init(a, tiles, kblocks, unit, units);
-            TcSeg sg;
+            walk.init(tiles, kblocks, unit, units, part, S);
             if (!PAIR && a.early) {
                 // weight tiles of this CTA's first segment go in flight before the wait; their partner tiles follow after it
                 TcWalk peek = walk;
-                if (peek.next(sg)) {
+                if (peek.next()) {
                     uint32_t mt, nt;
-                    tile_coords(sg.tile, m_tiles, n_tiles, mt, nt, a.group_m);
-                    for (uint32_t kb = sg.kb0; kb < sg.kb1 && pre < STAGES; ++kb, ++pre) {
+                    tile_coords(peek.tile, m_tiles, n_tiles, mt, nt, a.group_m);
+                    for (uint32_t kb = walk.kb0; kb < walk.kb1 && pre < STAGES; ++kb, ++pre) {
                         mbar_arrive_expect_tx(&full[pre], STAGE_BYTES);
                         uint8_t *st = smem + pre * STAGE_BYTES;
                         if (a.early == 1) load_a(st, kb, mt, &full[pre]);
@@ -252,10 +238,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             }
             pdl_wait();
             bool good = true;
-            while (good && walk.next(sg)) {
+            while (good && walk.next()) {
                 uint32_t mt, nt;
-                tile_coords(sg.tile, m_tiles, n_tiles, mt, nt, a.group_m);
-                for (uint32_t kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
+                tile_coords(walk.tile, m_tiles, n_tiles, mt, nt, a.group_m);
+                for (uint32_t kb = walk.kb0; kb < walk.kb1; ++kb, ++it) {
                     const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
                     uint8_t *st = smem + s * STAGE_BYTES;
                     if (it < pre) {// stage armed and half filled above
@@ -289,6 +275,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     load_b(st + A_BYTES, kb, nt, &full[s]);
                 }
             }
+            // a wait ran out: the copies in flight land before the block may go
+            if (!PAIR && !good)
+                for (uint32_t j = it < STAGES ? 0 : it - STAGES; j < it; ++j) mbar_wait(&full[j % STAGES], (j / STAGES) & 1u);
         }
     } else if (warp == 5) {
         if (lane == 0 && rank == 0) {
@@ -296,10 +285,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             uint32_t it = 0, local = 0;
             bool ok = true;
             TcWalk walk;
-            walk.init(a, tiles, kblocks, unit, units);
-            TcSeg sg;
-            for (; ok && walk.next(sg); ++local) {
-                const uint32_t buf = local & 1u, kb0 = sg.kb0, kb1 = sg.kb1;
+            walk.init(tiles, kblocks, unit, units, part, S);
+            for (; ok && walk.next(); ++local) {
+                const uint32_t buf = local & 1u, kb0 = walk.kb0, kb1 = walk.kb1;
                 if (!mbar_wait(&acc_empty[buf], ((local >> 1) & 1u) ^ 1u)) {
                     *failed = 4;
                     break;
@@ -340,7 +328,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         T *Y = static_cast<T *>(a.Y);
         const T *C = static_cast<const T *>(a.C);
         const bool c_rowmajor = C && a.c_col_stride == 1 && (a.c_row_stride % 8) == 0;
-        __shared__ int s_last;
+        if (S > 1) cluster_wait();
         // the all-reduce call this product feeds: its number stays put until the receiving kernel behind this one has run
         uint32_t ar_flag_v = 0;
         unsigned ar_q = 0;
@@ -437,172 +425,114 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         };
         uint32_t local = 0;
         TcWalk walk;
-        walk.init(a, tiles, kblocks, unit, units);
-        TcSeg sg;
+        walk.init(tiles, kblocks, unit, units, part, S);
         // hands an accumulator buffer back to the thread that issues the products (pair mode: in the even CTA)
         auto release_acc = [&](uint32_t buf) {
             if constexpr (PAIR) mbar_arrive_cluster(cluster_map(&acc_empty[buf], 0));
             else
                 mbar_arrive(&acc_empty[buf]);
         };
-        for (; walk.next(sg); ++local) {
-            uint32_t mt, nt;
-            const uint32_t tile = sg.tile, ks = sg.ord;
-            tile_coords(tile, m_tiles, n_tiles, mt, nt, a.group_m);
-            const uint32_t buf = local & 1u, m0 = PAIR ? (mt * 2 + rank) * TC_BM : mt * TC_BM, n0 = nt * BN;
-            if (!mbar_wait(&acc_full[buf], (local >> 1) & 1u)) {
-                *failed = 3;
-                break;
+        // Epilogue of columns [c_first, c_first + W) of this thread's row in the skinny forms, from their finished sums
+        auto finish = [&](const float *v, auto width, uint32_t mt, uint32_t row, uint32_t c_first) {
+            constexpr int W = decltype(width)::value;
+            if constexpr (PUSH) {
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    if (c_first + j < a.n) tc_push_value<T>(a, ar_flag_v, ar_q, row, c_first + j, a.alpha * v[j], row < a.m, lane);
+            } else if (a.swiglu) {
+                swiglu_rows(v, width, mt, c_first);
+            } else if (a.rope) {
+                rope_rows(v, width, mt, c_first);
+            } else if (row < a.m) {
+                // all of C before the first store: behind the stores of Y, which may be the same memory as far as the compiler knows,
+                // each load would wait for its own round trip
+                float add[W];
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    add[j] = C && c_first + j < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(c_first + j) * a.c_col_stride]) : 0.f;
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    if (c_first + j < a.n) {
+                        float o = a.alpha * v[j];
+                        if (C) o += a.beta * add[j];
+                        Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(c_first + j) * a.y_col_stride] = Num<T>::from_f(o);
+                    }
+                }
             }
+        };
+        // W columns per CTA of the cluster, WC of them at a time, from the receive buffer
+        auto finish_received = [&](auto chunk, const uint8_t *from, uint32_t W, uint32_t mt, uint32_t row, uint32_t c_first) {
+            constexpr int WC = decltype(chunk)::value;
+            const uint32_t trow = warp * 32 + lane;
+            for (uint32_t c = 0; c < W; c += WC) {
+                if (c_first + c >= a.n) break;// the same for every thread of the block
+                float v[WC];
+#pragma unroll
+                for (int j = 0; j < WC; ++j) v[j] = 0.f;
+                for (uint32_t src = 0; src < S; ++src) {
+#pragma unroll
+                    for (int g = 0; g < WC / 4; ++g) {
+                        const float4 x = *reinterpret_cast<const float4 *>(from + (((src * W + c) / 4 + g) * 128 + trow) * 16);
+                        v[4 * g] += x.x, v[4 * g + 1] += x.y, v[4 * g + 2] += x.z, v[4 * g + 3] += x.w;
+                    }
+                }
+                finish(v, chunk, mt, row, c_first + c);
+            }
+        };
+        bool ok = true;// after a wait that ran out nothing is waited for any more, but every barrier of the block is still met
+        for (; walk.next(); ++local) {
+            uint32_t mt, nt;
+            tile_coords(walk.tile, m_tiles, n_tiles, mt, nt, a.group_m);
+            const uint32_t buf = local & 1u, phase = (local >> 1) & 1u, m0 = PAIR ? (mt * 2 + rank) * TC_BM : mt * TC_BM, n0 = nt * BN;
+            const uint32_t row = m0 + warp * 32 + lane;
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], phase) ? 1 : 0);
+            if (!ok) *failed = 3;
             tc_fence_after();
-            if (sg.ncontrib > 1) {
-                // split-K: park this split's fp32 tile; the last split to arrive sums all of them in split order
-                const uint32_t trow = warp * 32 + lane;
-                float *mine = a.partial + (static_cast<size_t>(tile) * a.splits + ks) * (TC_BM * BN) + static_cast<size_t>(trow) * BN;
+            if constexpr (BN <= 64) {
+                if (S > 1) {
+                    const uint32_t W = BN / S, shift = __ffs(W) - 1, trow = warp * 32 + lane;// a power of two
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_cluster(&recv_free[buf], phase ^ 1u) ? 1 : 0);
+                    uint8_t *box = recv + buf * RECV_BYTES;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += 32) {
+                        uint32_t r[32];
+                        tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int g = 0; g < 8; ++g) {
+                            const uint32_t c = c0 + 4 * g, to = c >> shift;
+                            if (n0 + c < a.n)
+                                st_cluster_v4(cluster_map(box + (((part * W + (c & (W - 1))) / 4) * 128 + trow) * 16, to), r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+                        }
+                    }
+                    tc_fence_before();
+                    fence_cluster();
+                    __syncwarp();
+                    if (lane == 0) release_acc(buf);
+                    if (lane < S) mbar_arrive_cluster(cluster_map(&recv_full[buf], lane));
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_cluster(&recv_full[buf], phase) ? 1 : 0);
+                    if (!ok) *failed = 5;
+                    if (W >= 8) finish_received(std::integral_constant<int, 8>{}, box, W, mt, row, n0 + part * W);
+                    else
+                        finish_received(std::integral_constant<int, 4>{}, box, W, mt, row, n0 + part * W);
+                    __syncwarp();
+                    if (lane < S) mbar_arrive_cluster(cluster_map(&recv_free[buf], lane));
+                    continue;
+                }
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     uint32_t r[32];
                     tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
                     tmem_ld_wait();
+                    float v[32];
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4)
-                        *reinterpret_cast<uint4 *>(mine + c0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+                    finish(v, std::integral_constant<int, 32>{}, mt, row, n0 + c0);
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) release_acc(buf);
-                // the barrier orders the 128 threads' stores before thread 0's release-increment (cumulative at gpu scope)
-                asm volatile("bar.sync 2, 128;" ::: "memory");
-                if (threadIdx.x == 0) {
-                    unsigned old;
-                    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.counter + tile) : "memory");
-                    s_last = old == sg.ncontrib - 1 ? 1 : 0;
-                }
-                asm volatile("bar.sync 2, 128;" ::: "memory");
-                if (!s_last) continue;
-                const uint32_t row = m0 + trow;
-                const float *base = a.partial + static_cast<size_t>(tile) * a.splits * (TC_BM * BN) + static_cast<size_t>(trow) * BN;
-                if constexpr (BN <= 64) {// split-K is only planned for the skinny (swapped) shapes
-                    if (a.swiglu) {
-                        float acc[BN];
-#pragma unroll
-                        for (int c = 0; c < BN; ++c) acc[c] = 0.f;
-#pragma unroll 2
-                        for (uint32_t sidx = 0; sidx < sg.ncontrib; ++sidx) {
-                            const float4 *src = reinterpret_cast<const float4 *>(base + static_cast<size_t>(sidx) * (TC_BM * BN));
-                            float4 v[BN / 4];
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) v[c] = __ldcg(src + c);
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) acc[4 * c] += v[c].x, acc[4 * c + 1] += v[c].y, acc[4 * c + 2] += v[c].z, acc[4 * c + 3] += v[c].w;
-                        }
-                        swiglu_rows(acc, std::integral_constant<int, BN>{}, mt, n0);
-                    } else if (a.rope) {
-                        float acc[BN];
-#pragma unroll
-                        for (int c = 0; c < BN; ++c) acc[c] = 0.f;
-#pragma unroll 2
-                        for (uint32_t sidx = 0; sidx < sg.ncontrib; ++sidx) {
-                            const float4 *src = reinterpret_cast<const float4 *>(base + static_cast<size_t>(sidx) * (TC_BM * BN));
-                            float4 v[BN / 4];
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) v[c] = __ldcg(src + c);
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) acc[4 * c] += v[c].x, acc[4 * c + 1] += v[c].y, acc[4 * c + 2] += v[c].z, acc[4 * c + 3] += v[c].w;
-                        }
-                        rope_rows(acc, std::integral_constant<int, BN>{}, mt, n0);
-                    } else if (PUSH) {
-                        float acc[BN];
-#pragma unroll
-                        for (int c = 0; c < BN; ++c) acc[c] = 0.f;
-                        if (row < a.m) {
-#pragma unroll 2
-                            for (uint32_t sidx = 0; sidx < sg.ncontrib; ++sidx) {
-                                const float4 *src = reinterpret_cast<const float4 *>(base + static_cast<size_t>(sidx) * (TC_BM * BN));
-                                float4 v[BN / 4];
-#pragma unroll
-                                for (int c = 0; c < BN / 4; ++c) v[c] = __ldcg(src + c);
-#pragma unroll
-                                for (int c = 0; c < BN / 4; ++c) acc[4 * c] += v[c].x, acc[4 * c + 1] += v[c].y, acc[4 * c + 2] += v[c].z, acc[4 * c + 3] += v[c].w;
-                            }
-                        }
-#pragma unroll
-                        for (int c = 0; c < BN; ++c)
-                            if (n0 + c < a.n) tc_push_value<T>(a, ar_flag_v, ar_q, row, n0 + c, a.alpha * acc[c], row < a.m, lane);
-                    } else if (row < a.m) {
-                        // this thread's row of every split: the BN/4 loads of one split are independent, so the sum
-                        // costs one L2 round trip per split (fixed split order => deterministic)
-                        float4 acc[BN / 4];
-                        float add[BN];// this row of C: all loads in flight beside those of the sums (behind the stores of Y, which may
-                                      // be the same memory as far as the compiler knows, each would wait for its own round trip)
-#pragma unroll
-                        for (int c = 0; c < BN; ++c)
-                            add[c] = C && n0 + c < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(n0 + c) * a.c_col_stride]) : 0.f;
-#pragma unroll
-                        for (int c = 0; c < BN / 4; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-                        for (uint32_t sidx = 0; sidx < sg.ncontrib; ++sidx) {
-                            const float4 *src = reinterpret_cast<const float4 *>(base + static_cast<size_t>(sidx) * (TC_BM * BN));
-                            float4 v[BN / 4];
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) v[c] = __ldcg(src + c);
-#pragma unroll
-                            for (int c = 0; c < BN / 4; ++c) acc[c].x += v[c].x, acc[c].y += v[c].y, acc[c].z += v[c].z, acc[c].w += v[c].w;
-                        }
-#pragma unroll
-                        for (int c = 0; c < BN / 4; ++c) {
-                            const float vals[4] = {acc[c].x, acc[c].y, acc[c].z, acc[c].w};
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const uint32_t col = n0 + c * 4 + j;
-                                if (col < a.n) {
-                                    float v = a.alpha * vals[j];
-                                    if (C) v += a.beta * add[c * 4 + j];
-                                    Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(col) * a.y_col_stride] = Num<T>::from_f(v);
-                                }
-                            }
-                        }
-                    }
-                }
-                asm volatile("bar.sync 2, 128;" ::: "memory");
-                if (threadIdx.x == 0) a.counter[tile] = 0u;
                 continue;
-            }
-            const uint32_t row = m0 + warp * 32 + lane;
-            if constexpr (BN <= 64) {
-                if constexpr (PUSH) {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 32) {
-                        uint32_t r[32];
-                        tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (n0 + c0 + j < a.n) tc_push_value<T>(a, ar_flag_v, ar_q, row, n0 + c0 + j, a.alpha * __uint_as_float(r[j]), row < a.m, lane);
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) release_acc(buf);
-                    continue;
-                }
-                if (a.swiglu || a.rope) {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < BN; c0 += 32) {
-                        uint32_t r[32];
-                        tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
-                        tmem_ld_wait();
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-                        if (a.swiglu) swiglu_rows(v, std::integral_constant<int, 32>{}, mt, n0 + c0);
-                        else
-                            rope_rows(v, std::integral_constant<int, 32>{}, mt, n0 + c0);
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) release_acc(buf);
-                    continue;
-                }
             }
             if constexpr (BN == 256) {
                 if (a.swiglu) {
@@ -786,6 +716,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) cluster_sync();// the partner has read its accumulators and received every arrival meant for it
+    if (S > 1) {
+        if (warp >= 4) cluster_wait();// of the arrival at the start
+        cluster_sync();// every store and arrival meant for this CTA's shared memory has been made
+    }
     if (warp == 5) {
         tc_fence_after();
         if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
@@ -853,75 +787,32 @@ bool gemm_tc_supported(const rg_mat_mul_params *p, const void *const *in, void *
     return encode_fn() != nullptr;
 }
 
-// k-splits for a skinny product.  Stamps inside the kernel (16 tokens, 8192 x 1024 ... 7168 x 8192 weights) show where the time
-// goes: one CTA streams its operands at ~60 GB/s (its ring of stages in flight / the memory latency), and a split product pays
-// ~3 us more (partial tile to L2, release/acquire counter, the last arriver's sum) plus ~0.5 us per split summed.  The split
-// count minimises that estimate; products with more tiles than half the SMs only get a 2-way split when it repairs a mostly
-// empty last wave (22016 x 4096 at m = 16: 52.6 us unsplit, 46.6 / 52.8 / 88.9 us with 2 / 3 / 6 splits).
-static uint32_t tc_splits(uint32_t tiles, uint32_t kblocks) {
-    const uint32_t sms = static_cast<uint32_t>(sm_count());
-    const uint32_t cap = kblocks / 8 ? kblocks / 8 : 1;
-    if (tiles * 2 > sms) {
-        auto busy = [&](uint32_t items) { return static_cast<float>(items) / static_cast<float>((items + sms - 1) / sms * sms); };
-        // 96 tiles (12288 x 4096 at 32 tokens) leave a third of the SMs idle and two splits fill one wave and a third of the
-        // next; three fill two waves (batch-32 decode step 11.65 -> 11.55 ms)
-        if (cap >= 3 && tiles < sms && busy(3 * tiles) > busy(tiles) + 0.25f && busy(3 * tiles) > busy(2 * tiles) + 0.15f) return 3;
-        return (cap >= 2 && tiles < 2 * sms && busy(2 * tiles) > busy(tiles) + 0.15f) ? 2 : 1;
+// Skinny products (the tokens on the instruction's N side): up to 64 tokens against at least one tile of weight rows
+static bool tc_swapped(const rg_mat_mul_params *p) { return p->m <= 64 && p->n >= 128; }
+// CTAs of a cluster that share a tile: 1, 2, 4 or 8, whichever the model below says is done first.  A k-block (16 KiB of weights) takes an
+// SM 0.345 us when all of them stream and never less than 0.31; every round of tiles pays for what its exchange does not hide
+// behind the next tile's stream (about 4 us less 0.12 per k-block); launch and drain 3 us.  Measured at 8 tokens with
+// 1 / 2 / 4 / 8 CTAs: 4096 x 4096 21.4 / 13.6 / 11.7 / 14.3 us (model 22.8 / 13.1 / 10.1 / 14.4), 22016 x 4096 45.7 / 36.5 / 41.5 / 54.1 us,
+// 32000 x 1024 14.5 / 20.1 / 31.6 / 57.2 us, 57344 x 8192 174 / 156 / 151 / 193 us, 8192 x 28672 130 / 75 / 75 / 87 us.
+static uint32_t tc_ksplit(uint32_t tiles, uint32_t kblocks, const int (&clusters)[4]) {
+    if (const char *force = std::getenv("RG_B200_TC_KSPLIT")) {// tuning knob
+        const int f = std::atoi(force);
+        if ((f == 1 || f == 2 || f == 4 || f == 8) && static_cast<uint32_t>(f) <= kblocks && clusters[f == 1 ? 0 : f == 2 ? 1 : f == 4 ? 2 : 3] > 0) return static_cast<uint32_t>(f);
     }
-    uint32_t smax = sms / tiles;
-    if (smax > cap) smax = cap;
-    if (smax > 16) smax = 16;
-    const float tile_us = static_cast<float>(kblocks) * (TC_BM * TC_BK * 2) / 60000.f;// one CTA streaming a whole tile's k range
+    const float sms = static_cast<float>(sm_count());
     uint32_t best = 1;
-    float best_us = tile_us;
-    for (uint32_t s = 2; s <= smax; ++s) {
-        const float us = tile_us / static_cast<float>(s) + 3.0f + 0.5f * static_cast<float>(s);
+    float best_us = 1e30f;
+    for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t s = 1u << i, c = static_cast<uint32_t>(clusters[i]);
+        if (c == 0 || (s > 1 && s > kblocks)) continue;
+        const float rounds = static_cast<float>((tiles + c - 1) / c), busy = static_cast<float>((tiles < c ? tiles : c) * s) / sms;
+        const float kb = static_cast<float>((kblocks + s - 1) / s), kb_us = 0.345f * busy > 0.31f ? 0.345f * busy : 0.31f;
+        float seen = s > 1 ? 4.0f - 0.12f * kb : 0.f;
+        if (seen < 0.f) seen = 0.f;
+        const float us = rounds * (kb * kb_us + seen);
         if (us < best_us) best_us = us, best = s;
     }
     return best;
-}
-struct TcPlan {
-    bool swap;
-    uint32_t bn, tiles, splits;
-    uint32_t streamk_grid;// != 0: stream-K over this many CTAs; `splits` is then the partial slots per tile
-    size_t counter_bytes, partial_bytes;
-};
-static TcPlan tc_plan(const rg_mat_mul_params *p) {
-    TcPlan pl;
-    pl.swap = p->m <= 64 && p->n >= 128;
-    const uint32_t km = pl.swap ? p->n : p->m, kn = pl.swap ? p->m : p->n;
-    pl.bn = pl.swap ? (p->m <= 32 ? 32 : 64) : (p->n >= 256 ? 256 : 128);
-    pl.tiles = ((km + TC_BM - 1) / TC_BM) * ((kn + pl.bn - 1) / pl.bn);
-    const uint32_t kblocks = (p->k + TC_BK - 1) / TC_BK;
-    pl.splits = pl.swap ? tc_splits(pl.tiles, kblocks) : 1;
-    pl.streamk_grid = 0;
-    if (pl.swap) {// tuning knobs: RG_B200_TC_SPLITS=<n> forces the split count of skinny products, RG_B200_TC_STREAMK=0/1 the mode
-        static const char *force = std::getenv("RG_B200_TC_SPLITS");
-        static const char *sk = std::getenv("RG_B200_TC_STREAMK");
-        const uint32_t sms = static_cast<uint32_t>(sm_count());
-        const uint64_t units = static_cast<uint64_t>(pl.tiles) * kblocks;
-        // stream-K when every SM gets a run of at least 64 k-blocks (1 MiB of weights): below that the partial-tile round
-        // trips of up to two boundary tiles per CTA cost more than the imbalance they remove (measured at 16 / 32 tokens:
-        // 22016 x 4096, 74 k-blocks per SM: 44.5 -> 41.6 us; 8192 x 3584, 24 per SM: 17.8 -> 20.0 us; 7168 x 8192, 48: equal)
-        bool streamk = units / sms >= 64;
-        if (sk && sk[0]) streamk = sk[0] != '0' && units >= sms;
-        if (force && force[0]) {
-            const uint32_t f = static_cast<uint32_t>(std::atoi(force));
-            if (f >= 1) pl.splits = f > kblocks ? kblocks : f, streamk = false;
-        }
-        if (streamk) {
-            const uint32_t per = static_cast<uint32_t>(units / sms);// the shortest run
-            const uint32_t slots = (kblocks + per - 1) / per + 1;   // the most CTAs one tile can span
-            if (slots <= 8) pl.streamk_grid = sms, pl.splits = slots;// deeper tiles keep the uniform split (cheaper sums)
-        }
-    }
-    pl.counter_bytes = pl.splits > 1 ? (static_cast<size_t>(pl.tiles) * 4 + 255) / 256 * 256 : 0;
-    pl.partial_bytes = pl.splits > 1 ? static_cast<size_t>(pl.tiles) * pl.splits * TC_BM * pl.bn * 4 : 0;
-    return pl;
-}
-size_t gemm_tc_workspace(const rg_mat_mul_params *p) {
-    const TcPlan pl = tc_plan(p);
-    return pl.counter_bytes + pl.partial_bytes;
 }
 
 // Measured on one rank's share of a tensor-parallel-8 decode step (16 tokens, 80 layers, one GPU, no exchange; 9.55 ms):
@@ -935,19 +826,54 @@ size_t gemm_tc_workspace(const rg_mat_mul_params *p) {
 // waits for a free stage 41 % of the time.  Leaving the activation-tile loads out altogether (timing only): 41.3 us.  What is
 // left is the fill and drain of the memory pipeline around the dependency on the previous kernel (~10 us per launch): the
 // TMA-only stream has no such dependency, so its launches overlap.
+// As many clusters of `size` CTAs as the device holds at once (0 where it cannot say)
+template<class... K>
+static int tc_resident_clusters(void (*kern)(K...), unsigned size, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(sm_count()) / size * size), cfg.blockDim = dim3(TC_THREADS), cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 0) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return n;
+}
 template<class T, int BN, int STAGES, bool PUSH = false, bool MN = false>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &a_in, cudaStream_t st) {
     TcArgs a = a_in;
     a.group_m = TC_GROUP_M;
-    constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
+    constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 2 * tc_recv_bytes(BN) + (2 * STAGES + 8) * 8 + 16 + 1024;
     auto kern = gemm_tc_kernel<T, BN, STAGES, PUSH, false, MN>;
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     // the whole shared-memory carve-out, so that a CTA of the next kernel can sit beside one of this kernel when both fit
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, static_cast<int>(cudaSharedmemCarveoutMaxShared)));
-    const uint32_t items = ((a.n + BN - 1) / BN) * ((a.m + TC_BM - 1) / TC_BM) * a.splits;
-    const uint32_t sms = static_cast<uint32_t>(sm_count());
-    const uint32_t grid = a.streamk ? a.streamk : (items < sms ? items : sms);
-    RG_CHECK_CUDA(launch_pdl(kern, dim3(grid), dim3(TC_THREADS), smem, st, ma, mb, a));
+    const uint32_t tiles = ((a.n + BN - 1) / BN) * ((a.m + TC_BM - 1) / TC_BM), sms = static_cast<uint32_t>(sm_count());
+    a.ksplit = 1;
+    if constexpr (BN <= 64) {
+        static int clusters[64][4] = {};// per device and cluster size 1, 2, 4, 8; asked once
+        int dev = 0;
+        RG_CHECK_CUDA(cudaGetDevice(&dev));
+        int here[4] = {static_cast<int>(sms), 0, 0, 0};
+        if (dev >= 0 && dev < 64) {
+            if (clusters[dev][0] == 0) {
+                for (int i = 3; i >= 1; --i) clusters[dev][i] = tc_resident_clusters(kern, 1u << i, smem);
+                clusters[dev][0] = static_cast<int>(sms);
+            }
+            for (int i = 0; i < 4; ++i) here[i] = clusters[dev][i];
+        }
+        a.ksplit = tc_ksplit(tiles, (a.k + TC_BK - 1) / TC_BK, here);
+        if (a.ksplit > 1) {
+            const uint32_t c = static_cast<uint32_t>(here[a.ksplit == 2 ? 1 : a.ksplit == 4 ? 2 : 3]);
+            RG_CHECK_CUDA(launch_pdl_cluster(kern, dim3((tiles < c ? tiles : c) * a.ksplit), dim3(TC_THREADS), smem, st, a.ksplit, ma, mb, a));
+            count_launch();
+            return launch_status();
+        }
+    }
+    RG_CHECK_CUDA(launch_pdl(kern, dim3(tiles < sms ? tiles : sms), dim3(TC_THREADS), smem, st, ma, mb, a));
     count_launch();
     return launch_status();
 }
@@ -963,7 +889,7 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     constexpr int BN = 256, STAGES = 6;
     TcArgs a = a_in;
     a.group_m = TC_GROUP_M;// of 256-row tiles; measured on 8192 x 12288 x 4096: 4 / 8 / 16 / 32 row tiles per group 577 / 557 / 550 / 605 us
-    constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + (BN / 2) * TC_BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
+    constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + (BN / 2) * TC_BK * 2) + (2 * STAGES + 8) * 8 + 16 + 1024;
     auto kern = gemm_tc_kernel<T, BN, STAGES, false, true, MN>;
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const uint32_t items = ((a.n + BN - 1) / BN) * ((a.m + 2 * TC_BM - 1) / (2 * TC_BM));
@@ -972,18 +898,8 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     int dev = 0;
     RG_CHECK_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && resident[dev] == 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(sm_count()) & ~1u), cfg.blockDim = dim3(TC_THREADS), cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr, cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-            cudaGetLastError();
-            n = sm_count() / 2;
-        }
-        resident[dev] = n;
+        const int n = tc_resident_clusters(kern, 2, smem);
+        resident[dev] = n > 0 ? n : sm_count() / 2;
     }
     const uint32_t pairs = static_cast<uint32_t>(dev >= 0 && dev < 64 ? resident[dev] : sm_count() / 2);
     const uint32_t grid = 2 * (items < pairs ? items : pairs);
@@ -992,11 +908,9 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     return launch_status();
 }
 
-int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
+int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     const int is_bf16 = p->dtype == RG_BF16;
     const size_t es = 2;
-    const TcPlan pl = tc_plan(p);
-    if (pl.splits > 1 && !ws) return RG_ERR_NULL;
     const bool mn = !p->trans_b;
     auto map_b = [&](CUtensorMap *map, const void *base, uint32_t box_rows) {
         return mn ? make_map_mn(map, base, is_bf16, p->k, p->n) : make_map(map, base, is_bf16, p->n, p->k, p->k, box_rows);
@@ -1008,12 +922,9 @@ int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *c
         const uint8_t *C = p->has_bias ? static_cast<const uint8_t *>(in[2]) + b * p->stride_c * es : nullptr;
         TcArgs a = {};
         a.alpha = p->alpha, a.beta = p->beta, a.is_bf16 = is_bf16, a.k = p->k;
-        a.splits = pl.splits, a.streamk = pl.streamk_grid;
-        a.counter = static_cast<unsigned *>(ws);
-        a.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + pl.counter_bytes);
         CUtensorMap ma, mb;
         // a skinny activation matrix (m <= 64) goes on the N side of the instruction: D^T[n, m] = W[n,k] X[m,k]^T
-        const bool swap = pl.swap;
+        const bool swap = tc_swapped(p);
         uint32_t bn;
         if (!swap) {
             bn = p->n >= 256 ? 256 : 128;
@@ -1021,7 +932,7 @@ int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *c
             a.early = (p->flags & RG_MM_B_STATIC) ? 2u : 0u;
             a.Y = Y, a.y_row_stride = p->n, a.y_col_stride = 1;
             a.C = C, a.c_row_stride = p->bias_row_stride, a.c_col_stride = p->bias_col_stride;
-            if (bn == 256 && pl.splits == 1 && !pl.streamk_grid && p->m >= 512 && tc_pair_enabled()) {
+            if (bn == 256 && p->m >= 512 && tc_pair_enabled()) {
                 if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !map_b(&mb, B, 128)) return RG_ERR_CUDA;
                 const int rc = mn ? (is_bf16 ? tc_launch_pair<__nv_bfloat16, true>(ma, mb, a, st) : tc_launch_pair<__half, true>(ma, mb, a, st))
                                   : (is_bf16 ? tc_launch_pair<__nv_bfloat16>(ma, mb, a, st) : tc_launch_pair<__half>(ma, mb, a, st));
@@ -1040,7 +951,7 @@ int gemm_tc(const rg_mat_mul_params *p, void *ws, const void *const *in, void *c
         int rc;
 #define RG_TC(T, MN)                                                                                                           \
     (bn == 256 ? tc_launch<T, 256, 4, false, MN>(ma, mb, a, st) : bn == 128 ? tc_launch<T, 128, 6, false, MN>(ma, mb, a, st) \
-     : bn == 64 ? tc_launch<T, 64, 8, false, MN>(ma, mb, a, st) : tc_launch<T, 32, 8, false, MN>(ma, mb, a, st))
+     : bn == 64 ? tc_launch<T, 64, 6, false, MN>(ma, mb, a, st) : tc_launch<T, 32, 8, false, MN>(ma, mb, a, st))
         rc = mn ? (is_bf16 ? RG_TC(__nv_bfloat16, true) : RG_TC(__half, true)) : (is_bf16 ? RG_TC(__nv_bfloat16, false) : RG_TC(__half, false));
 #undef RG_TC
         if (rc != RG_OK) return rc;
@@ -1061,7 +972,7 @@ int gemm_tc_qkv_rope(const rg_linear_params *p, const void *const *in, void *con
     const int is_bf16 = p->dtype == RG_BF16;
     TcArgs a = {};
     a.alpha = 1.f, a.beta = 0.f, a.is_bf16 = is_bf16, a.k = p->k, a.m = p->m, a.n = p->n;
-    a.splits = 1, a.early = 2;
+    a.early = 2;
     a.Y = out[0], a.y_row_stride = p->n, a.y_col_stride = 1;
     a.rope = 1, a.nq = nq, a.tokens_per_seq = p->tokens_per_seq, a.log2_theta = log2f(p->theta);
     a.pos = static_cast<const int64_t *>(in[4]), a.table = static_cast<const int32_t *>(in[5]);
@@ -1077,103 +988,71 @@ int gemm_tc_qkv_rope(const rg_linear_params *p, const void *const *in, void *con
 // pairs 128 gate rows with their 128 up rows, so both halves of an output column meet in one accumulator.
 // Up to 64 tokens: the weights go on the instruction's M side (a tile = 64 gate rows + their 64 up rows), the tokens on its N
 // side, with the k-split / stream-K plan of the plain skinny product; the up half of a tile hands its sums to the gate half.
-static rg_mat_mul_params swiglu_small_as_mat_mul(const rg_linear_params *p) {
-    rg_mat_mul_params mp = {};
-    mp.dtype = p->dtype, mp.m = p->m, mp.n = p->n, mp.k = p->k, mp.batch = 1;
-    mp.trans_b = 1, mp.alpha = 1.f, mp.flags = RG_MM_B_STATIC;
-    return mp;
-}
 bool gemm_tc_swiglu_small_shape(const rg_linear_params *p) {
     return (p->dtype == RG_FP16 || p->dtype == RG_BF16) && p->epilogue == 2 && p->prologue == 0 && p->m > 4 && p->m <= 64 &&
            p->n % 128 == 0 && p->n >= 128 && p->k % 8 == 0 && p->k >= 64 && encode_fn() != nullptr;
 }
-size_t gemm_tc_swiglu_small_workspace(const rg_linear_params *p) {
-    const rg_mat_mul_params mp = swiglu_small_as_mat_mul(p);
-    return gemm_tc_workspace(&mp);
-}
-int gemm_tc_swiglu_small(const rg_linear_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
+int gemm_tc_swiglu_small(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     if (!gemm_tc_swiglu_small_shape(p)) return RG_ERR_SHAPE;
     if (!in[0] || !in[1] || !out[0]) return RG_ERR_NULL;
     if (!aligned16(in[0]) || !aligned16(in[1]) || !aligned16(out[0])) return RG_ERR_ALIGN;
-    const rg_mat_mul_params mp = swiglu_small_as_mat_mul(p);
-    const TcPlan pl = tc_plan(&mp);
-    if (!pl.swap) return RG_ERR_SHAPE;
-    if (pl.splits > 1 && !ws) return RG_ERR_NULL;
     const int is_bf16 = p->dtype == RG_BF16;
     TcArgs a = {};
     a.alpha = 1.f, a.beta = 0.f, a.is_bf16 = is_bf16, a.k = p->k;
     a.m = p->n, a.n = p->m;// kernel rows = weight rows (gate and up interleaved by tile), kernel columns = tokens
-    a.splits = pl.splits, a.streamk = pl.streamk_grid;
-    a.counter = static_cast<unsigned *>(ws);
-    a.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + pl.counter_bytes);
     a.early = 1, a.swiglu = p->n / 2;
     a.Y = out[0], a.y_row_stride = 1, a.y_col_stride = p->n / 2;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, 64) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, pl.bn)) return RG_ERR_CUDA;
-    if (pl.bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8>(ma, mb, a, st) : tc_launch<__half, 32, 8>(ma, mb, a, st);
-    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 8>(ma, mb, a, st) : tc_launch<__half, 64, 8>(ma, mb, a, st);
+    const uint32_t bn = p->m <= 32 ? 32 : 64;
+    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, 64) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, bn)) return RG_ERR_CUDA;
+    if (bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8>(ma, mb, a, st) : tc_launch<__half, 32, 8>(ma, mb, a, st);
+    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 6>(ma, mb, a, st) : tc_launch<__half, 64, 6>(ma, mb, a, st);
 }
 
 // Row-parallel product feeding an all-reduce: the plain skinny product (weights on the M side) whose epilogue stores into the
 // communicator's slots.  m <= 64 tokens, n a multiple of 8, no C operand.
-int gemm_tc_push(const rg_mat_mul_params *p, void *ws, const void *const *in, const ArPeers &peers, cudaStream_t st) {
+int gemm_tc_push(const rg_mat_mul_params *p, const void *const *in, const ArPeers &peers, cudaStream_t st) {
     if (p->dtype != RG_FP16 && p->dtype != RG_BF16) return RG_ERR_UNSUPPORTED;
     if (p->trans_a || !p->trans_b || p->batch != 1 || p->has_bias || p->m == 0 || p->m > 64 || p->n < 128 || p->n % 8 != 0 || p->k % 8 != 0 || p->k < 64)
         return RG_ERR_UNSUPPORTED;
     if (!aligned16(in[0]) || !aligned16(in[1]) || !encode_fn()) return RG_ERR_UNSUPPORTED;
-    const TcPlan pl = tc_plan(p);
-    if (!pl.swap) return RG_ERR_UNSUPPORTED;
-    if (pl.splits > 1 && !ws) return RG_ERR_NULL;
     const int is_bf16 = p->dtype == RG_BF16;
     TcArgs a = {};
     a.alpha = p->alpha, a.beta = 0.f, a.is_bf16 = is_bf16, a.k = p->k;
     a.m = p->n, a.n = p->m;// kernel rows = output features, kernel columns = tokens
-    a.splits = pl.splits, a.streamk = pl.streamk_grid;
-    a.counter = static_cast<unsigned *>(ws);
-    a.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + pl.counter_bytes);
     a.early = (p->flags & RG_MM_B_STATIC) ? 1u : 0u;
     a.push = peers.two_shot ? 2u : 1u, a.ar = peers;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, TC_BM) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, pl.bn)) return RG_ERR_CUDA;
-    if (pl.bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8, true>(ma, mb, a, st) : tc_launch<__half, 32, 8, true>(ma, mb, a, st);
-    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 8, true>(ma, mb, a, st) : tc_launch<__half, 64, 8, true>(ma, mb, a, st);
+    const uint32_t bn = p->m <= 32 ? 32 : 64;
+    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, TC_BM) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, bn)) return RG_ERR_CUDA;
+    if (bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8, true>(ma, mb, a, st) : tc_launch<__half, 32, 8, true>(ma, mb, a, st);
+    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 6, true>(ma, mb, a, st) : tc_launch<__half, 64, 6, true>(ma, mb, a, st);
 }
 
 // The same for the QKV projection with its split / rotation / cache-append epilogue on 5..64 tokens (a 128-row tile = one head).
-static rg_mat_mul_params qkv_small_as_mat_mul(const rg_linear_params *p) { return swiglu_small_as_mat_mul(p); }
 bool gemm_tc_qkv_rope_small_shape(const rg_linear_params *p) {
     const uint32_t nq = p->n_heads, nkv = p->kv.n_kv_heads;
     return (p->dtype == RG_FP16 || p->dtype == RG_BF16) && p->epilogue == 3 && p->prologue == 0 && p->m > 4 && p->m <= 64 && p->kv.head_dim == 128 &&
            nq > 0 && nkv > 0 && p->n == (nq + 2 * nkv) * 128u && p->k % 8 == 0 && p->k >= 64 && p->theta > 0.f && encode_fn() != nullptr;
 }
-size_t gemm_tc_qkv_rope_small_workspace(const rg_linear_params *p) {
-    const rg_mat_mul_params mp = qkv_small_as_mat_mul(p);
-    return gemm_tc_workspace(&mp);
-}
-int gemm_tc_qkv_rope_small(const rg_linear_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
+int gemm_tc_qkv_rope_small(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     if (!gemm_tc_qkv_rope_small_shape(p)) return RG_ERR_SHAPE;
     if (!in[0] || !in[1] || !in[4] || !out[0] || !out[1] || !out[2]) return RG_ERR_NULL;
     if (in[5] && p->kv.page_size == 0) return RG_ERR_SHAPE;
     if (!aligned16(in[0]) || !aligned16(in[1])) return RG_ERR_ALIGN;
-    const rg_mat_mul_params mp = qkv_small_as_mat_mul(p);
-    const TcPlan pl = tc_plan(&mp);
-    if (!pl.swap) return RG_ERR_SHAPE;
-    if (pl.splits > 1 && !ws) return RG_ERR_NULL;
     const int is_bf16 = p->dtype == RG_BF16;
     TcArgs a = {};
     a.alpha = 1.f, a.beta = 0.f, a.is_bf16 = is_bf16, a.k = p->k;
     a.m = p->n, a.n = p->m;// kernel rows = output features (a tile = a head), kernel columns = tokens
-    a.splits = pl.splits, a.streamk = pl.streamk_grid;
-    a.counter = static_cast<unsigned *>(ws);
-    a.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + pl.counter_bytes);
     a.early = 1;
     a.rope = 1, a.nq = p->n_heads, a.tokens_per_seq = p->tokens_per_seq, a.log2_theta = log2f(p->theta);
     a.pos = static_cast<const int64_t *>(in[4]), a.table = static_cast<const int32_t *>(in[5]);
     a.q_out = out[0], a.kc = out[1], a.vc = out[2], a.kv = p->kv;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, TC_BM) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, pl.bn)) return RG_ERR_CUDA;
-    if (pl.bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8>(ma, mb, a, st) : tc_launch<__half, 32, 8>(ma, mb, a, st);
-    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 8>(ma, mb, a, st) : tc_launch<__half, 64, 8>(ma, mb, a, st);
+    const uint32_t bn = p->m <= 32 ? 32 : 64;
+    if (!make_map(&ma, in[1], is_bf16, p->n, p->k, p->k, TC_BM) || !make_map(&mb, in[0], is_bf16, p->m, p->k, p->k, bn)) return RG_ERR_CUDA;
+    if (bn == 32) return is_bf16 ? tc_launch<__nv_bfloat16, 32, 8>(ma, mb, a, st) : tc_launch<__half, 32, 8>(ma, mb, a, st);
+    return is_bf16 ? tc_launch<__nv_bfloat16, 64, 6>(ma, mb, a, st) : tc_launch<__half, 64, 6>(ma, mb, a, st);
 }
 
 int gemm_tc_swiglu(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st) {
@@ -1187,7 +1066,7 @@ int gemm_tc_swiglu(const rg_linear_params *p, const void *const *in, void *const
     const int is_bf16 = p->dtype == RG_BF16;
     TcArgs a = {};
     a.alpha = 1.f, a.beta = 0.f, a.is_bf16 = is_bf16, a.k = p->k, a.m = p->m, a.n = p->n;
-    a.splits = 1, a.early = 2, a.swiglu = f;
+    a.early = 2, a.swiglu = f;
     a.Y = out[0], a.y_row_stride = f, a.y_col_stride = 1;
     CUtensorMap ma, mb;
     if (!make_map(&ma, in[0], is_bf16, p->m, p->k, p->k, TC_BM) || !make_map(&mb, in[1], is_bf16, p->n, p->k, p->k, 128)) return RG_ERR_CUDA;

@@ -429,15 +429,14 @@ static bool linear_is_skinny(const rg_linear_params *p) {
 }
 size_t rg_b200_linear_workspace(const rg_linear_params *p) {
     if (!p) return 0;
-    if (linear_is_tc_swiglu_small(p)) return gemm_tc_swiglu_small_workspace(p);
-    if (linear_is_tc_qkv_small(p)) return gemm_tc_qkv_rope_small_workspace(p);
+    if (linear_is_tc_swiglu_small(p) || linear_is_tc_qkv_small(p)) return 0;
     if (!linear_is_skinny(p)) return 0;
     return linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->epilogue, &p->kv, p->n_heads);
 }
 int rg_b200_linear(const rg_linear_params *p, void *ws, const void *const *in, void *const *out, void *stream) {
     if (!p || !in || !out) return RG_ERR_NULL;
-    if (linear_is_tc_swiglu_small(p)) return gemm_tc_swiglu_small(p, ws, in, out, static_cast<cudaStream_t>(stream));
-    if (linear_is_tc_qkv_small(p)) return gemm_tc_qkv_rope_small(p, ws, in, out, static_cast<cudaStream_t>(stream));
+    if (linear_is_tc_swiglu_small(p)) return gemm_tc_swiglu_small(p, in, out, static_cast<cudaStream_t>(stream));
+    if (linear_is_tc_qkv_small(p)) return gemm_tc_qkv_rope_small(p, in, out, static_cast<cudaStream_t>(stream));
     if (linear_is_skinny(p)) {
         SkinnyCall c = {};
         c.dtype = p->dtype, c.m = p->m, c.n = p->n, c.k = p->k, c.epilogue = p->epilogue;

@@ -54,16 +54,11 @@ static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *i
 extern "C" {
 
 size_t rg_b200_mat_mul_workspace(const rg_mat_mul_params *p) {
-    // the tensor-core kernel's split-K path and the skinny kernel's k-split need scratch; sized for whichever could be chosen
+    // the fp32 tensor-core kernel's and the skinny kernel's k-split need scratch
     if (!p || p->m == 0 || p->n == 0 || p->k == 0 || p->batch == 0) return 0;
     if (p->dtype == RG_F32) return gemm_tc32_preferred(p) || (p->force_kernel == 5 && !p->trans_a) ? gemm_tc32_workspace(p) : 0;
     if ((p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a) return 0;
-    size_t bytes = gemm_tc_workspace(p);
-    if (skinny_shape(p)) {
-        const size_t s = linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0);
-        bytes = s > bytes ? s : bytes;
-    }
-    return bytes;
+    return skinny_shape(p) ? linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0) : 0;
 }
 
 int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, void *stream) {
@@ -78,7 +73,7 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         case 0: break;
         case 1: return gemm_simt(p, in, out, st);
         case 2: return gemv_shape(p) ? run_gemv(p, in, out, st) : RG_ERR_UNSUPPORTED;
-        case 3: return gemm_tc_supported(p, in, out) ? gemm_tc(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
+        case 3: return gemm_tc_supported(p, in, out) ? gemm_tc(p, in, out, st) : RG_ERR_UNSUPPORTED;
         case 4: return skinny_shape(p) ? run_skinny(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
         case 5: return gemm_tc32(p, ws, in, out, st);
         default: return RG_ERR_UNSUPPORTED;
@@ -93,7 +88,7 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         const int rc = run_skinny(p, ws, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;
     }
-    if (gemm_tc_supported(p, in, out) && (ws || gemm_tc_workspace(p) == 0)) return gemm_tc(p, ws, in, out, st);
+    if (gemm_tc_supported(p, in, out)) return gemm_tc(p, in, out, st);
     return gemm_simt(p, in, out, st);
 }
 }

@@ -119,6 +119,22 @@ def test_skinny_swapped_operands(dtype, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", HALF)
+@pytest.mark.parametrize("trans_b", [True, False])
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 64), (8, 520, 128), (9, 520, 200), (32, 256, 512), (33, 1024, 1024), (64, 1280, 8192), (48, 12288, 4096), (3, 5000, 4096)])
+def test_skinny_clusters_share_a_tile(dtype, trans_b, m, n, k):
+    """k divided over clusters of 1, 2, 4 and 8 CTAs, several tiles per cluster, ragged tiles and tokens; integer data is exact in
+    fp32 accumulation whatever the order of the sums."""
+    rng = np.random.default_rng(m + n + k)
+    a, b, c = (rng.integers(-2, 3, s).astype(np.float32) for s in ((m, k), (k, n), (m, n)))
+    bd = ops.dev(b.T.copy() if trans_b else b).to(dtype)
+    want = torch.from_numpy(a @ b + 2 * c).to(dtype)
+    for _ in range(2):
+        y = ops.mat_mul(ops.dev(a).to(dtype), bd, ops.dev(c).to(dtype), trans_b=trans_b, beta=2.0, force=3)
+        assert _ok()
+        assert torch.equal(y.cpu(), want)
+
+
+@pytest.mark.parametrize("dtype", HALF)
 @pytest.mark.parametrize("m,n,k,residual", [(16, 22016, 4096, False), (32, 32000, 4096, True), (8, 20000, 4104, False)])
 def test_skinny_stream_k(dtype, m, n, k, residual):
     """Skinny products with at least 64 k-blocks per SM run in stream-K mode: every CTA owns one contiguous run of
