@@ -908,6 +908,24 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     return launch_status();
 }
 
+// Tile of the products of more than 64 tokens: 128 x 256 on single CTAs, 256 x 256 on pairs (512 tokens and more) or 128 x 128.  L2 bounds
+// all three (10 to 12 TB/s into shared memory), so the smaller tile takes 0.6 of the time of the 128 x 256 one instead of half, and a
+// pair 0.88; the smaller wins where the large ones leave SMs idle.  Small / large / pair: 333 x 4096 x 4096 with residual 25.2 / 32.6 / 29.5 us,
+// 333 x 4096 x 11008 59.5 / 74.1 / 62.3, 333 x 12288 x 4096 46.0 / 40.7 / 52.3, 700 x 4096 x 4096 43.9 / 33.5 / 31.1, 1500 x 4096 x 4096
+// 64.1 / 56.4 / 50.4.
+enum : int { TC_TILE_128, TC_TILE_256, TC_TILE_PAIR };
+static int tc_wide_tile(uint32_t m, uint32_t n) {
+    if (n < 256) return TC_TILE_128;
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    auto rounds = [](uint64_t tiles, uint32_t slots) { return static_cast<float>((tiles + slots - 1) / slots); };
+    auto up = [](uint32_t v, uint32_t t) { return static_cast<uint64_t>((v + t - 1) / t); };
+    const float small = 0.6f * rounds(up(m, 128) * up(n, 128), sms), large = rounds(up(m, 128) * up(n, 256), sms);
+    const bool pairs = m >= 512 && tc_pair_enabled();
+    const float pair = pairs ? 0.88f * rounds(up(m, 256) * up(n, 256), sms / 2) : 1e30f;
+    if (pair <= large && pair <= small) return TC_TILE_PAIR;
+    return small < large ? TC_TILE_128 : TC_TILE_256;
+}
+
 int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     const int is_bf16 = p->dtype == RG_BF16;
     const size_t es = 2;
@@ -927,12 +945,13 @@ int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out,
         const bool swap = tc_swapped(p);
         uint32_t bn;
         if (!swap) {
-            bn = p->n >= 256 ? 256 : 128;
+            const int tile = tc_wide_tile(p->m, p->n);
+            bn = tile == TC_TILE_128 ? 128 : 256;
             a.m = p->m, a.n = p->n;
             a.early = (p->flags & RG_MM_B_STATIC) ? 2u : 0u;
             a.Y = Y, a.y_row_stride = p->n, a.y_col_stride = 1;
             a.C = C, a.c_row_stride = p->bias_row_stride, a.c_col_stride = p->bias_col_stride;
-            if (bn == 256 && p->m >= 512 && tc_pair_enabled()) {
+            if (tile == TC_TILE_PAIR) {
                 if (!make_map(&ma, A, is_bf16, p->m, p->k, p->k, TC_BM) || !map_b(&mb, B, 128)) return RG_ERR_CUDA;
                 const int rc = mn ? (is_bf16 ? tc_launch_pair<__nv_bfloat16, true>(ma, mb, a, st) : tc_launch_pair<__half, true>(ma, mb, a, st))
                                   : (is_bf16 ? tc_launch_pair<__nv_bfloat16>(ma, mb, a, st) : tc_launch_pair<__half>(ma, mb, a, st));
