@@ -15,8 +15,13 @@
 // i / j innermost (K-major or MN-major in shared memory; nothing is transposed).  Roles of the warps:
 //   converters  eight warps (two such groups on alternate k-blocks for up to 32 rows, a form bound by the weights' stream):
 //               16-byte loads one k-block ahead in registers, three 16-byte stores per eight values into the swizzled planes
-//   issuer      one thread, 24 tcgen05.mma (kind::f16, 128 x BN x 16) per 64 values of k
-//   drainers    add the large product's accumulator (double-buffered) to registers after every 64 values of k
+//   drainers    add the large product's accumulator (double-buffered) to registers after every 64 values of k; one thread of the
+//               first issues the 24 tcgen05.mma (kind::f16, 128 x BN x 16) of the k-block after the one it is about to drain (a
+//               seventeenth warp for that would take a quarter of everybody's registers; the skinny forms have it)
+// FAST: rows on 16 bytes and k, and n where it is innermost, multiples of 8.  Addresses are then 32-bit offsets kept per item, rows past the
+// edge repeat the last one (they only reach results that are not stored) and only the last k-block looks at the end of k.  With
+// bounds and addresses worked out per piece the converters executed twice the instructions and set the pace: 509 x 2752 x 1024 45.3 us then,
+// 38.4 now; 509 x 32000 x 1024 281 and 235 (142 TFLOP/s); the prompt above 1.79 -> 1.61 ms
 // k is split between CTAs where tiles are few; the last to arrive adds the parked sums in order.
 // Measured against the 64 x 64 CUDA-core tiles: a 509-token prompt through four layers of width 1024 with a 32000-word head
 // (86 GFLOP) 5.74 -> 2.06 ms, a 32-token prompt through two layers of width 256 446 -> 237 us.
@@ -32,7 +37,8 @@ constexpr int T3_BM = 128, T3_BK = 64;
 template<int BN> struct Tc32Shape {
     static constexpr int STAGES = BN == 128 ? 2 : 3, GROUPS = BN == 32 ? 2 : 1, CONV = 8 * GROUPS, EPI = BN == 128 ? 8 : 4;
     static constexpr int COLS = BN * 4 / EPI;// accumulator columns of a drainer thread
-    static constexpr int THREADS = (CONV + EPI + 1) * 32;
+    static constexpr bool ISSUER = BN != 128;// a warp of its own for the thread that issues the products
+    static constexpr int THREADS = (CONV + EPI + (ISSUER ? 1 : 0)) * 32;
     static constexpr uint32_t P_TILE = T3_BM * T3_BK * 2, Q_TILE = BN * T3_BK * 2, STAGE = 3 * (P_TILE + Q_TILE);
     static constexpr size_t SMEM = STAGES * STAGE + (2 * STAGES + 6) * 8 + 16 + 1024;
 };
@@ -110,10 +116,10 @@ struct Tc32Walk {
     }
 };
 
-template<int BN, bool P_MN, bool Q_MN>
+template<int BN, bool P_MN, bool Q_MN, bool FAST>
 __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(const __grid_constant__ Tc32Args a) {
     using Sh = Tc32Shape<BN>;
-    constexpr int STAGES = Sh::STAGES, GROUPS = Sh::GROUPS, CONV = Sh::CONV, EPI = Sh::EPI, COLS = Sh::COLS;
+    constexpr int STAGES = Sh::STAGES, GROUPS = Sh::GROUPS, EPI = Sh::EPI, COLS = Sh::COLS;
     constexpr uint32_t P_TILE = Sh::P_TILE, Q_TILE = Sh::Q_TILE, STAGE = Sh::STAGE;
     constexpr int NP = T3_BM * T3_BK / 8 / 256, NQ = BN * T3_BK / 8 / 256;// pieces of eight values per converter thread and k-block
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -135,7 +141,7 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
         *failed = 0;
         fence_mbar_init();
     }
-    if (warp == CONV + EPI) {
+    if (warp == EPI) {
         tmem_alloc(tmem_slot, 4 * BN);
         tmem_relinquish();
     }
@@ -147,28 +153,53 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
     Tc32Walk w;
     w.item = blockIdx.x;
 
-    if (warp >= EPI && warp < EPI + CONV) {
+    if (warp >= EPI && warp < EPI + Sh::CONV) {
         // ---- converters ----
         const uint32_t group = (warp - EPI) / 8, t = threadIdx.x - EPI * 32 - group * 256;
         // piece c of a tile: K-major (row, 8 k) = (c / 8, c % 8); MN-major (k, 8 rows) = (c / (rows / 8), c % (rows / 8))
+        uint32_t offp[NP], offq[NQ];// FAST: offsets of this thread's pieces from the k-block's first element
+        auto aim = [&]() {
+            if constexpr (FAST) {
+                auto offset = [&](const Tc32Operand &o, bool mn, uint32_t rows, uint32_t tile, int i) {
+                    const uint32_t c = t + i * 256;
+                    if (mn) {
+                        const uint32_t col = tile * rows + c % (rows / 8) * 8;
+                        return c / (rows / 8) * o.ld + (col < o.inner ? col : o.inner - 8);
+                    }
+                    const uint32_t row = tile * rows + c / 8;
+                    return (row < o.outer ? row : o.outer - 1) * o.ld + c % 8 * 8;
+                };
+#pragma unroll
+                for (int i = 0; i < NP; ++i) offp[i] = offset(a.p, P_MN, T3_BM, w.mt, i);
+#pragma unroll
+                for (int i = 0; i < NQ; ++i) offq[i] = offset(a.q, Q_MN, BN, w.nt, i);
+            }
+        };
         auto fetch = [&](float (&v)[NP + NQ][8], int i) {
-            const uint32_t c = t + (i < NP ? i : i - NP) * 256;
-            if (i < NP) {
-                const float *base = a.p.x + w.b * a.p.stride;
-                if (P_MN) tc32_load(a.p, base, w.kb * T3_BK + c / (T3_BM / 8), w.mt * T3_BM + c % (T3_BM / 8) * 8, v[i]);
-                else
-                    tc32_load(a.p, base, w.mt * T3_BM + c / 8, w.kb * T3_BK + c % 8 * 8, v[i]);
+            const bool first = i < NP, mn = first ? P_MN : Q_MN;
+            const uint32_t c = t + (first ? i : i - NP) * 256, rows = first ? T3_BM : BN, tile = first ? w.mt : w.nt;
+            const Tc32Operand &o = first ? a.p : a.q;
+            const float *base = o.x + w.b * o.stride;
+            if constexpr (FAST) {
+                const float4 *src = reinterpret_cast<const float4 *>(base + (mn ? static_cast<uint64_t>(w.kb * T3_BK) * o.ld : w.kb * T3_BK) + (first ? offp[i] : offq[i - NP]));
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+                if ((w.kb + 1) * T3_BK <= a.k) {// the same for every thread
+                    x = __ldg(src), y = __ldg(src + 1);
+                } else if (w.kb * T3_BK + (mn ? c / (rows / 8) : c % 8 * 8) < a.k) {
+                    x = __ldg(src), y = __ldg(src + 1);
+                }
+                v[i][0] = x.x, v[i][1] = x.y, v[i][2] = x.z, v[i][3] = x.w, v[i][4] = y.x, v[i][5] = y.y, v[i][6] = y.z, v[i][7] = y.w;
             } else {
-                const float *base = a.q.x + w.b * a.q.stride;
-                if (Q_MN) tc32_load(a.q, base, w.kb * T3_BK + c / (BN / 8), w.nt * BN + c % (BN / 8) * 8, v[i]);
+                if (mn) tc32_load(o, base, w.kb * T3_BK + c / (rows / 8), tile * rows + c % (rows / 8) * 8, v[i]);
                 else
-                    tc32_load(a.q, base, w.nt * BN + c / 8, w.kb * T3_BK + c % 8 * 8, v[i]);
+                    tc32_load(o, base, tile * rows + c / 8, w.kb * T3_BK + c % 8 * 8, v[i]);
             }
         };
         bool more = w.open(a, kblocks), ok = true;
         for (uint32_t g = 0; more && g < group; ++g) more = w.next(a, kblocks);
         float v[NP + NQ][8];
         if (more) {
+            aim();
 #pragma unroll
             for (int i = 0; i < NP + NQ; ++i) fetch(v, i);
         }
@@ -179,7 +210,9 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
                 *failed = 1;
                 break;
             }
+            const uint32_t item = w.item;
             for (int g = 0; more && g < GROUPS; ++g) more = w.next(a, kblocks);// the block fetched while this one is converted
+            if (more && w.item != item) aim();
             uint8_t *st = smem + s * STAGE;
 #pragma unroll
             for (int i = 0; i < NP + NQ; ++i) {
@@ -201,50 +234,56 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
         }
-    } else if (warp == CONV + EPI) {
-        // ---- issuer ----
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(1, T3_BM, BN) | (P_MN ? 1u << 15 : 0u) | (Q_MN ? 1u << 16 : 0u);
-            uint32_t local = 0, d_small = 0;
-            bool more = w.open(a, kblocks);
-            for (uint32_t it = 0; more; ++it) {
-                const uint32_t s = it % STAGES, buf = it & 1u, d_big = tmem + buf * BN;
-                const bool fresh = w.kb == w.kb0;
-                if (fresh) {
-                    d_small = tmem + (2 + (local & 1u)) * BN;
-                    if (!mbar_wait(&small_empty[local & 1u], ((local >> 1) & 1u) ^ 1u)) {
-                        *failed = 2;
-                        break;
-                    }
-                    ++local;
-                }
-                if (!mbar_wait(&big_empty[buf], ((it >> 1) & 1u) ^ 1u) || !mbar_wait(&full[s], (it / STAGES) & 1u)) {
-                    *failed = 3;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t ps = smem_u32(smem + s * STAGE), qs = ps + 3 * P_TILE;
-                auto product = [&](uint32_t d, uint32_t pp, uint32_t qp, bool first) {
-#pragma unroll
-                    for (uint32_t kk = 0; kk < T3_BK / 16; ++kk) {
-                        const uint32_t pt = ps + pp * P_TILE, qt = qs + qp * Q_TILE;
-                        const uint64_t pd = P_MN ? smem_desc_sw128_mn(pt + kk * 2048, T3_BK * 128) : smem_desc_sw128(pt + kk * 32);
-                        const uint64_t qd = Q_MN ? smem_desc_sw128_mn(qt + kk * 2048, T3_BK * 128) : smem_desc_sw128(qt + kk * 32);
-                        tc_mma_f16(d, pd, qd, idesc, first && kk == 0 ? 0u : 1u);
-                    }
-                };
-                product(d_big, 0, 0, true);
-                product(d_small, 0, 2, fresh);
-                product(d_small, 2, 0, false);
-                product(d_small, 1, 1, false);
-                product(d_small, 0, 1, false);
-                product(d_small, 1, 0, false);
-                tc_commit(&empty[s]);
-                tc_commit(&big_full[buf]);
-                more = w.next(a, kblocks);
-            }
-        }
     } else {
+        // the products of the next k-block of this CTA's schedule (one thread)
+        Tc32Walk wi = w;
+        uint32_t issued = 0, items_issued = 0, d_small = 0;
+        bool to_issue = warp == (Sh::ISSUER ? EPI + Sh::CONV : 0) && lane == 0 && wi.open(a, kblocks);
+        auto issue = [&]() {
+            const uint32_t idesc = instr_desc(1, T3_BM, BN) | (P_MN ? 1u << 15 : 0u) | (Q_MN ? 1u << 16 : 0u);
+            const uint32_t s = issued % STAGES, buf = issued & 1u, d_big = tmem + buf * BN;
+            const bool fresh = wi.kb == wi.kb0;
+            bool good = true;
+            if (fresh) {
+                d_small = tmem + (2 + (items_issued & 1u)) * BN;
+                good = mbar_wait(&small_empty[items_issued & 1u], ((items_issued >> 1) & 1u) ^ 1u);
+                ++items_issued;
+            }
+            good = good && mbar_wait(&big_empty[buf], ((issued >> 1) & 1u) ^ 1u) && mbar_wait(&full[s], (issued / STAGES) & 1u);
+            if (!good) {
+                *failed = 3;
+                to_issue = false;
+                return;
+            }
+            tc_fence_after();
+            const uint32_t ps = smem_u32(smem + s * STAGE), qs = ps + 3 * P_TILE;
+            auto product = [&](uint32_t d, uint32_t pp, uint32_t qp, bool first) {
+#pragma unroll
+                for (uint32_t kk = 0; kk < T3_BK / 16; ++kk) {
+                    const uint32_t pt = ps + pp * P_TILE, qt = qs + qp * Q_TILE;
+                    const uint64_t pd = P_MN ? smem_desc_sw128_mn(pt + kk * 2048, T3_BK * 128) : smem_desc_sw128(pt + kk * 32);
+                    const uint64_t qd = Q_MN ? smem_desc_sw128_mn(qt + kk * 2048, T3_BK * 128) : smem_desc_sw128(qt + kk * 32);
+                    tc_mma_f16(d, pd, qd, idesc, first && kk == 0 ? 0u : 1u);
+                }
+            };
+            product(d_big, 0, 0, true);
+            product(d_small, 0, 2, fresh);
+            product(d_small, 2, 0, false);
+            product(d_small, 1, 1, false);
+            product(d_small, 0, 1, false);
+            product(d_small, 1, 0, false);
+            tc_commit(&empty[s]);
+            tc_commit(&big_full[buf]);
+            ++issued;
+            to_issue = wi.next(a, kblocks);
+        };
+        if constexpr (Sh::ISSUER) {
+            while (to_issue) issue();
+            if (warp >= EPI) w.item = a.tiles * a.splits;// nothing to drain
+        } else if (to_issue) {
+            issue();
+        }
+        __syncwarp();
         // ---- drainers: warp w reads the tensor-memory lanes of quarter w % 4 (tile rows), COLS columns of them ----
         const uint32_t quarter = warp & 3u, col = (warp >> 2) * COLS, trow = quarter * 32 + lane, lanes = (quarter * 32u) << 16;
         uint32_t it = 0, local = 0;
@@ -256,6 +295,10 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
             const uint32_t item = w.item, tile = item / a.splits, mt = w.mt, nt = w.nt, b = w.b;
             for (uint32_t kb = w.kb0; kb < w.kb1; ++kb, ++it) {
                 const uint32_t buf = it & 1u;
+                if constexpr (!Sh::ISSUER) {
+                    if (to_issue) issue();
+                    __syncwarp();
+                }
                 ok = ok && t3_warp_wait(&big_full[buf], (it >> 1) & 1u);
                 tc_fence_after();
 #pragma unroll
@@ -334,7 +377,7 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == CONV + EPI) {
+    if (warp == EPI) {
         tc_fence_after();
         tmem_dealloc(tmem, 4 * BN);
     }
@@ -375,9 +418,9 @@ size_t gemm_tc32_workspace(const rg_mat_mul_params *p) {
     return pl.counter_bytes + pl.partial_bytes;
 }
 
-template<int BN, bool P_MN, bool Q_MN>
+template<int BN, bool P_MN, bool Q_MN, bool FAST>
 static int tc32_launch(const Tc32Args &a, cudaStream_t st) {
-    auto kern = gemm_tc32_kernel<BN, P_MN, Q_MN>;
+    auto kern = gemm_tc32_kernel<BN, P_MN, Q_MN, FAST>;
     constexpr size_t smem = Tc32Shape<BN>::SMEM;
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const uint32_t items = a.tiles * a.splits, sms = static_cast<uint32_t>(sm_count());
@@ -404,9 +447,13 @@ int gemm_tc32(const rg_mat_mul_params *p, void *ws, const void *const *in, void 
     a.y_i = pl.swap ? 1 : p->n, a.y_j = pl.swap ? p->n : 1;
     a.c_i = pl.swap ? p->bias_col_stride : p->bias_row_stride, a.c_j = pl.swap ? p->bias_row_stride : p->bias_col_stride;
     a.alpha = p->alpha, a.beta = p->beta;
-    if (!pl.swap) return p->trans_b ? tc32_launch<128, false, false>(a, st) : tc32_launch<128, false, true>(a, st);
-    if (pl.bn == 32) return p->trans_b ? tc32_launch<32, false, false>(a, st) : tc32_launch<32, true, false>(a, st);
-    return p->trans_b ? tc32_launch<64, false, false>(a, st) : tc32_launch<64, true, false>(a, st);
+    const auto small = [](const Tc32Operand &o) { return static_cast<uint64_t>(o.outer + 128) * o.ld < (1ull << 31); };
+    const bool fast = oa.vec && ob.vec && p->k % 8 == 0 && (p->trans_b || p->n % 8 == 0) && small(oa) && small(ob);
+#define RG_TC32(BN, P_MN, Q_MN) (fast ? tc32_launch<BN, P_MN, Q_MN, true>(a, st) : tc32_launch<BN, P_MN, Q_MN, false>(a, st))
+    if (!pl.swap) return p->trans_b ? RG_TC32(128, false, false) : RG_TC32(128, false, true);
+    if (pl.bn == 32) return p->trans_b ? RG_TC32(32, false, false) : RG_TC32(32, true, false);
+    return p->trans_b ? RG_TC32(64, false, false) : RG_TC32(64, true, false);
+#undef RG_TC32
 }
 
 int gemm_tc32_error_word(bool clear) { return error_symbol(s_tc32_error, clear); }
