@@ -10,6 +10,13 @@ static bool gemv_shape(const rg_mat_mul_params *p) {
            !p->has_bias && p->alpha == 1.0f && p->k % 8 == 0 && p->k * 2u <= 32768u;
 }
 
+// The streaming kernel multiplies on the CUDA cores: one or two rows keep up with HBM (5.1-5.4 TB/s on large weights), three and four do
+// not (3.5), while the tensor cores pay about 3 us more per launch.  At four rows: 4096 x 4096 11.0 us here, 11.6 there; 12288 x
+// 4096 29.2 and 23.2; 22016 x 4096 50.9 and 36.5.  The line lies at 20 million weights.
+static bool gemv_preferred(const rg_mat_mul_params *p) {
+    return gemv_shape(p) && (p->m <= 2 || static_cast<uint64_t>(p->n) * p->k < 20000000ull);
+}
+
 static int run_gemv(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     rg_linear_params lp = {};
     lp.dtype = p->dtype;
@@ -79,7 +86,7 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         default: return RG_ERR_UNSUPPORTED;
     }
     if (p->dtype == RG_F32) return gemm_tc32_preferred(p) ? gemm_tc32(p, ws, in, out, st) : gemm_simt(p, in, out, st);
-    if (gemv_shape(p) && aligned16(in[0]) && aligned16(in[1])) {
+    if (gemv_preferred(p) && aligned16(in[0]) && aligned16(in[1])) {
         const int rc = run_gemv(p, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;
     }
