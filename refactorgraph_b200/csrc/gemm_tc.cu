@@ -122,7 +122,9 @@ struct TcWalk {
 // shares each tile, every CTA streaming its part of k.  CTA r finishes columns (tokens) [r W, r W + W), W = BN / ksplit: the others
 // store their sums of those columns into its receive buffer over distributed shared memory (st.shared::cluster, counted on its
 // recv_full mbarrier; recv_free, counted on the senders', hands the buffer back), it adds them in rank order and runs the
-// epilogue of its W columns.  Two receive buffers, so the exchange of a tile overlaps the stream of the next.
+// epilogue of its W columns.  Two receive buffers, so the exchange of a tile overlaps the stream of the next.  The wide forms do the
+// same for products with fewer tiles than SMs, one tile per cluster: the receive buffer is then the ring itself, and
+// recv_free says that all CTAs have read their last stage.
 // Measured with stream-K / parked partial sums in global memory before: 8 tokens x 4096 x 4096 16.4 -> 11.6 us, 4096 x 11008 24.9 ->
 // 19.8, 12288 x 4096 26.6 -> 23.2, 22016 x 4096 37.7 -> 36.5, 32000 x 4096 49.4 -> 47.1; an 8-layer 7B step of 8 sequences 1.37 -> 1.17 ms.
 //
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     constexpr uint32_t ROWS = PAIR ? 2 * TC_BM : TC_BM;// rows of a tile
     constexpr bool MN_A = MN && BN <= 64, MN_B = MN && BN > 64;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;// 0 = the CTA that issues the products
-    const uint32_t S = PAIR || BN > 64 ? 1u : a.ksplit, part = S > 1 ? cluster_ctarank() : 0u;
+    const uint32_t S = PAIR ? 1u : a.ksplit, part = S > 1 ? cluster_ctarank() : 0u;
     const uint32_t unit = PAIR ? blockIdx.x >> 1 : blockIdx.x / S, units = PAIR ? gridDim.x >> 1 : gridDim.x / S;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // the swizzled tiles need 1024-byte alignment
@@ -652,60 +654,111 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             // tile of 128 x 256 took 12 us longer than the plain product with a load in front of every store.
             const bool rows_wide = a.y_col_stride == 1 && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor);
             Vec16<T> cnext[4];
-            auto fetch_c = [&](int c0) {
-                if (C && rows_wide && row < a.m && n0 + c0 + 32 <= a.n) {
-                    const T *csrc = C + static_cast<uint64_t>(row) * a.c_row_stride + n0 + c0;
+            auto fetch_c = [&](uint32_t col0) {
+                if (C && rows_wide && row < a.m && col0 + 32 <= a.n) {
+                    const T *csrc = C + static_cast<uint64_t>(row) * a.c_row_stride + col0;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) cnext[j].load(csrc + 8 * j);
                 }
             };
-            fetch_c(0);
+            auto store_columns = [&](const float (&r)[32], const Vec16<T> (&cv)[4], uint32_t col0) {
+                if (row >= a.m) return;
+                if (rows_wide && col0 + 32 <= a.n) {
+                    // contiguous 64-byte run of this thread's row: four 16-byte stores
+                    T *dst = Y + static_cast<uint64_t>(row) * a.y_row_stride + col0;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 8) {
+                        float f[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) f[e] = a.alpha * r[j + e];
+                        if (C) {
+                            float cf[8];
+                            cv[j / 8].unpack(cf);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) f[e] += a.beta * cf[e];
+                        }
+                        Vec16<T> v;
+                        v.pack(f);
+                        v.store(dst + j);
+                    }
+                } else {
+                    float add[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const uint32_t col = col0 + j;
+                        add[j] = C && col < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]) : 0.f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const uint32_t col = col0 + j;
+                        if (col < a.n) {
+                            float v = a.alpha * r[j];
+                            if (C) v += a.beta * add[j];
+                            Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(col) * a.y_col_stride] = Num<T>::from_f(v);
+                        }
+                    }
+                }
+            };
+            if constexpr (BN > 64 && !PAIR) {
+                if (S > 1) {
+                    const uint32_t W = BN / S, shift = __ffs(W) - 1, trow = warp * 32 + lane, mine = n0 + part * W;// W: 32, 64 or 128
+                    if (lane < S) mbar_arrive_cluster(cluster_map(&recv_free[0], lane));// this CTA's products are done: its ring may be written
+                    fetch_c(mine);
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_cluster(&recv_free[0], 0) ? 1 : 0);
+                    if (!ok) {
+                        *failed = 5;
+                        continue;// nothing is stored into a ring that may still be in use
+                    }
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += 32) {
+                        uint32_t r[32];
+                        tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
+                        tmem_ld_wait();
+                        if (n0 + c0 >= a.n) break;
+                        const uint32_t to = cluster_map(smem + ((part * W + (c0 & (W - 1))) / 4 * 128 + trow) * 16, c0 >> shift);
+#pragma unroll
+                        for (int g = 0; g < 8; ++g) st_cluster_v4(to + g * 2048, r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+                    }
+                    fence_cluster();
+                    __syncwarp();
+                    if (lane < S) mbar_arrive_cluster(cluster_map(&recv_full[0], lane));
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait_cluster(&recv_full[0], 0) ? 1 : 0);
+                    if (!ok) *failed = 5;
+                    for (uint32_t c = 0; c < W && mine + c < a.n; c += 32) {
+                        Vec16<T> cv[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) cv[j] = cnext[j];
+                        if (c + 32 < W) fetch_c(mine + c + 32);
+                        float v[32];
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+                        for (uint32_t src = 0; src < S; ++src) {
+                            const float4 *from = reinterpret_cast<const float4 *>(smem) + ((src * W + c) / 4 * 128 + trow);
+#pragma unroll
+                            for (int g = 0; g < 8; ++g) {
+                                const float4 x = from[g * 128];
+                                v[4 * g] += x.x, v[4 * g + 1] += x.y, v[4 * g + 2] += x.z, v[4 * g + 3] += x.w;
+                            }
+                        }
+                        store_columns(v, cv, mine + c);
+                    }
+                    continue;
+                }
+            }
+            fetch_c(n0);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t r[32];
                 Vec16<T> cv[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) cv[j] = cnext[j];
-                if (c0 + 32 < BN) fetch_c(c0 + 32);
+                if (c0 + 32 < BN) fetch_c(n0 + c0 + 32);
                 tmem_ld_32x32(tmem_base + buf * BN + ((warp * 32u) << 16) + c0, r);
                 tmem_ld_wait();
-                if (row < a.m) {
-                    if (rows_wide && n0 + c0 + 32 <= a.n) {
-                        // contiguous 64-byte run of this thread's row: four 16-byte stores
-                        T *dst = Y + static_cast<uint64_t>(row) * a.y_row_stride + n0 + c0;
+                float v[32];
 #pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            float f[8];
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) f[e] = a.alpha * __uint_as_float(r[j + e]);
-                            if (C) {
-                                float cf[8];
-                                cv[j / 8].unpack(cf);
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) f[e] += a.beta * cf[e];
-                            }
-                            Vec16<T> v;
-                            v.pack(f);
-                            v.store(dst + j);
-                        }
-                    } else {
-                        float add[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const uint32_t col = n0 + c0 + j;
-                            add[j] = C && col < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]) : 0.f;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const uint32_t col = n0 + c0 + j;
-                            if (col < a.n) {
-                                float v = a.alpha * __uint_as_float(r[j]);
-                                if (C) v += a.beta * add[j];
-                                Y[static_cast<uint64_t>(row) * a.y_row_stride + static_cast<uint64_t>(col) * a.y_col_stride] = Num<T>::from_f(v);
-                            }
-                        }
-                    }
-                }
+                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+                store_columns(v, cv, n0 + c0);
             }
             // hand the accumulator buffer back to the MMA warp
             tc_fence_before();
@@ -815,6 +868,26 @@ static uint32_t tc_ksplit(uint32_t tiles, uint32_t kblocks, const int (&clusters
     return best;
 }
 
+// The wide forms: clusters share a tile only where every tile has one to itself, at least four k-blocks and 32 columns per CTA.  Shared
+// memory fills at 64 bytes a cycle, which makes a k-block 0.33 us (128 columns) or 0.43 us (256); launch and drain 4 us, exchange 3 us.
+static float tc_wide_us(uint32_t tiles, uint32_t kblocks, uint32_t bn, uint32_t s, uint32_t slots) {
+    const float kb_us = bn > 128 ? 0.43f : 0.33f, crowd = bn > 128 ? 0.57f : 0.33f;// 144 CTAs of the large tile share what L2 delivers
+    const uint32_t busy = tiles * s < slots ? tiles * s : slots;
+    const float us = busy * 2 > slots ? kb_us + (crowd - kb_us) * (2.f * busy / slots - 1.f) : kb_us;
+    return 4.f + static_cast<float>((static_cast<uint64_t>(tiles) * s + slots - 1) / slots) * static_cast<float>((kblocks + s - 1) / s) * us + (s > 1 ? 3.f : 0.f);
+}
+static uint32_t tc_ksplit_wide(uint32_t tiles, uint32_t kblocks, uint32_t bn, const int (&clusters)[4]) {
+    uint32_t best = 1;
+    float best_us = tc_wide_us(tiles, kblocks, bn, 1, static_cast<uint32_t>(sm_count()));
+    for (uint32_t i = 1; i < 4; ++i) {
+        const uint32_t s = 1u << i;
+        if (s * 4 > kblocks || s * 32 > bn || static_cast<int>(tiles) > clusters[i]) continue;
+        const float us = tc_wide_us(tiles, kblocks, bn, s, static_cast<uint32_t>(sm_count()));
+        if (us < best_us) best_us = us, best = s;
+    }
+    return best;
+}
+
 // Measured on one rank's share of a tensor-parallel-8 decode step (16 tokens, 80 layers, one GPU, no exchange; 9.55 ms):
 // 5 stages for the up-to-32-token products, so that a CTA of the next kernel fits beside one of this kernel and fetches its
 // first weight tiles early: 10.55 ms; 10 stages: 9.57 ms; asking L2 for 16 / 48 further weight tiles of the CTA's run before the
@@ -852,26 +925,26 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs 
     // the whole shared-memory carve-out, so that a CTA of the next kernel can sit beside one of this kernel when both fit
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, static_cast<int>(cudaSharedmemCarveoutMaxShared)));
     const uint32_t tiles = ((a.n + BN - 1) / BN) * ((a.m + TC_BM - 1) / TC_BM), sms = static_cast<uint32_t>(sm_count());
-    a.ksplit = 1;
-    if constexpr (BN <= 64) {
-        static int clusters[64][4] = {};// per device and cluster size 1, 2, 4, 8; asked once
-        int dev = 0;
-        RG_CHECK_CUDA(cudaGetDevice(&dev));
-        int here[4] = {static_cast<int>(sms), 0, 0, 0};
-        if (dev >= 0 && dev < 64) {
-            if (clusters[dev][0] == 0) {
-                for (int i = 3; i >= 1; --i) clusters[dev][i] = tc_resident_clusters(kern, 1u << i, smem);
-                clusters[dev][0] = static_cast<int>(sms);
-            }
-            for (int i = 0; i < 4; ++i) here[i] = clusters[dev][i];
+    static int clusters[64][4] = {};// per device and cluster size 1, 2, 4, 8; asked once
+    int dev = 0;
+    RG_CHECK_CUDA(cudaGetDevice(&dev));
+    int here[4] = {static_cast<int>(sms), 0, 0, 0};
+    if (dev >= 0 && dev < 64) {
+        if (clusters[dev][0] == 0) {
+            for (int i = 3; i >= 1; --i) clusters[dev][i] = tc_resident_clusters(kern, 1u << i, smem);
+            clusters[dev][0] = static_cast<int>(sms);
         }
-        a.ksplit = tc_ksplit(tiles, (a.k + TC_BK - 1) / TC_BK, here);
-        if (a.ksplit > 1) {
-            const uint32_t c = static_cast<uint32_t>(here[a.ksplit == 2 ? 1 : a.ksplit == 4 ? 2 : 3]);
-            RG_CHECK_CUDA(launch_pdl_cluster(kern, dim3((tiles < c ? tiles : c) * a.ksplit), dim3(TC_THREADS), smem, st, a.ksplit, ma, mb, a));
-            count_launch();
-            return launch_status();
-        }
+        for (int i = 0; i < 4; ++i) here[i] = clusters[dev][i];
+    }
+    const uint32_t kblocks = (a.k + TC_BK - 1) / TC_BK;
+    if constexpr (BN <= 64) a.ksplit = tc_ksplit(tiles, kblocks, here);
+    else
+        a.ksplit = a.rope || a.swiglu ? 1u : tc_ksplit_wide(tiles, kblocks, BN, here);
+    if (a.ksplit > 1) {
+        const uint32_t c = static_cast<uint32_t>(here[a.ksplit == 2 ? 1 : a.ksplit == 4 ? 2 : 3]);
+        RG_CHECK_CUDA(launch_pdl_cluster(kern, dim3((tiles < c ? tiles : c) * a.ksplit), dim3(TC_THREADS), smem, st, a.ksplit, ma, mb, a));
+        count_launch();
+        return launch_status();
     }
     RG_CHECK_CUDA(launch_pdl(kern, dim3(tiles < sms ? tiles : sms), dim3(TC_THREADS), smem, st, ma, mb, a));
     count_launch();
@@ -908,21 +981,29 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     return launch_status();
 }
 
-// Tile of the products of more than 64 tokens: 128 x 256 on single CTAs, 256 x 256 on pairs (512 tokens and more) or 128 x 128.  L2 bounds
-// all three (10 to 12 TB/s into shared memory), so the smaller tile takes 0.6 of the time of the 128 x 256 one instead of half, and a
-// pair 0.88; the smaller wins where the large ones leave SMs idle.  Small / large / pair: 333 x 4096 x 4096 with residual 25.2 / 32.6 / 29.5 us,
-// 333 x 4096 x 11008 59.5 / 74.1 / 62.3, 333 x 12288 x 4096 46.0 / 40.7 / 52.3, 700 x 4096 x 4096 43.9 / 33.5 / 31.1, 1500 x 4096 x 4096
-// 64.1 / 56.4 / 50.4.
+// Tile of the products of more than 64 tokens: 128 x 256 on single CTAs, 256 x 256 on pairs (512 tokens and more) or 128 x 128, whichever
+// tc_wide_us says is done first.  Shared memory fills at 64 bytes a cycle and SM and L2 delivers 10 to 12 TB/s in all, so the
+// smaller tile costs more per product; it wins where the large ones leave SMs idle.  128 / 256 columns / pair with residual, the
+// first two with the split they get: 333 x 4096 x 4096 26.1 / 22.0 / 29.8 us (30.4 unsplit), 333 x 4096 x 11008 60.5 / 44.3 / 62.9 (70.5),
+// 333 x 12288 x 4096 47.8 / 39.8 / 52.9, 128 x 4096 x 4096 15.1 / 17.9 / 29.5, 300 x 1024 x 2752 12.0 / 15.1 / 22.0 (18.0 and 22.3 unsplit),
+// 700 x 4096 x 4096 44.7 / 30.9 / 31.6, 2000 x 10240 x 8192 367 / 281 / 256.
 enum : int { TC_TILE_128, TC_TILE_256, TC_TILE_PAIR };
-static int tc_wide_tile(uint32_t m, uint32_t n) {
+static int tc_wide_tile(uint32_t m, uint32_t n, uint32_t k) {
     if (n < 256) return TC_TILE_128;
-    const uint32_t sms = static_cast<uint32_t>(sm_count());
-    auto rounds = [](uint64_t tiles, uint32_t slots) { return static_cast<float>((tiles + slots - 1) / slots); };
-    auto up = [](uint32_t v, uint32_t t) { return static_cast<uint64_t>((v + t - 1) / t); };
-    const float small = 0.6f * rounds(up(m, 128) * up(n, 128), sms), large = rounds(up(m, 128) * up(n, 256), sms);
-    const bool pairs = m >= 512 && tc_pair_enabled();
-    const float pair = pairs ? 0.88f * rounds(up(m, 256) * up(n, 256), sms / 2) : 1e30f;
-    if (pair <= large && pair <= small) return TC_TILE_PAIR;
+    const uint32_t sms = static_cast<uint32_t>(sm_count()), kblocks = (k + TC_BK - 1) / TC_BK;
+    auto up = [](uint32_t v, uint32_t t) { return (v + t - 1) / t; };
+    // clusters that the device is sure to hold at once: one CTA in nine is left over where SMs do not divide evenly
+    const int clusters[4] = {static_cast<int>(sms), static_cast<int>(sms / 2), static_cast<int>(sms * 8 / 9 / 4), static_cast<int>(sms * 7 / 9 / 8)};
+    auto us = [&](uint32_t bn) {
+        const uint32_t tiles = up(m, 128) * up(n, bn);
+        return tc_wide_us(tiles, kblocks, bn, tc_ksplit_wide(tiles, kblocks, bn, clusters), sms);
+    };
+    const float small = us(128), large = us(256);
+    if (m >= 512 && tc_pair_enabled()) {
+        const uint64_t pairs = static_cast<uint64_t>(up(m, 256)) * up(n, 256);
+        const float pair = 4.f + static_cast<float>((pairs + sms / 2 - 1) / (sms / 2)) * static_cast<float>(kblocks) * 0.385f;
+        if (pair <= large && pair <= small) return TC_TILE_PAIR;
+    }
     return small < large ? TC_TILE_128 : TC_TILE_256;
 }
 
@@ -945,7 +1026,7 @@ int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out,
         const bool swap = tc_swapped(p);
         uint32_t bn;
         if (!swap) {
-            const int tile = tc_wide_tile(p->m, p->n);
+            const int tile = tc_wide_tile(p->m, p->n, p->k);
             bn = tile == TC_TILE_128 ? 128 : 256;
             a.m = p->m, a.n = p->n;
             a.early = (p->flags & RG_MM_B_STATIC) ? 2u : 0u;

@@ -135,6 +135,21 @@ def test_skinny_clusters_share_a_tile(dtype, trans_b, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", HALF)
+@pytest.mark.parametrize("trans_b", [True, False])
+@pytest.mark.parametrize("m,n,k", [(65, 136, 2048), (100, 1024, 1024), (128, 256, 8192), (300, 2752, 1024), (333, 4096, 1024), (511, 1000, 520), (600, 520, 512)])
+def test_wide_clusters_share_a_tile(dtype, trans_b, m, n, k):
+    """More than 64 tokens and fewer tiles than SMs: k divided over clusters, the sums exchanged through the ring; exact integer data,
+    ragged edges, residual and bias row."""
+    rng = np.random.default_rng(m + n + k)
+    a, b, c, r = (rng.integers(-2, 3, s).astype(np.float32) for s in ((m, k), (k, n), (m, n), (n,)))
+    bd = ops.dev(b.T.copy() if trans_b else b).to(dtype)
+    for add in (c, r, c):
+        y = ops.mat_mul(ops.dev(a).to(dtype), bd, ops.dev(add).to(dtype), trans_b=trans_b, beta=2.0, force=3)
+        assert _ok()
+        assert torch.equal(y.cpu(), torch.from_numpy(a @ b + 2 * add).to(dtype))
+
+
+@pytest.mark.parametrize("dtype", HALF)
 @pytest.mark.parametrize("m,n,k,residual", [(16, 22016, 4096, False), (32, 32000, 4096, True), (8, 20000, 4104, False)])
 def test_skinny_stream_k(dtype, m, n, k, residual):
     """Skinny products with at least 64 k-blocks per SM run in stream-K mode: every CTA owns one contiguous run of
