@@ -105,6 +105,7 @@ struct Phase {
     const uint8_t *W;  // weights (linear phases)
     uint32_t n, k;     // rows, columns of W
     uint32_t g, segs;  // rows per segment, segments per unit
+    uint32_t ng;       // groups of consumer threads that share the rows of a unit (narrow layers)
     uint32_t units;
     uint32_t layer;
 };
@@ -114,11 +115,18 @@ __host__ __device__ inline uint32_t pow2_floor_d(uint32_t v) {
     for (uint32_t b = 1; b && b <= v; b <<= 1) p = b;
     return p;
 }
-// Rows per segment (g) and units of a linear phase with `n` rows of `k` columns; one definition for the kernel's schedule and
-// for the host-side check that no CTA gets more units of a phase than its shared-memory partial-sum table holds.
-__host__ __device__ inline uint32_t mega_phase_units(int type, uint32_t n, uint32_t k, uint32_t segs, uint32_t D, uint32_t F, uint32_t &g_out) {
+// Groups that the 256 consumer threads form for rows of k columns: a row of up to 1024 columns (128 16-byte chunks) occupies only part
+// of them, so 2, 4 or 8 groups take four rows of the unit each.
+__host__ __device__ inline uint32_t mega_groups(uint32_t k) {
+    const uint32_t chunks = k / 8;
+    return chunks <= 32 ? 8 : chunks <= 64 ? 4 : chunks <= 128 ? 2 : 1;
+}
+// Rows per segment (g) and units of a linear phase with `n` rows of `k` columns, at most `most` rows a unit; one definition for the
+// kernel's schedule and for the host-side check that no CTA gets more units of a phase than its shared-memory partial-sum table holds
+// (the table takes 4 rows x 8 warps a unit, which is also 4 groups rows x 8 / groups warps).
+__host__ __device__ inline uint32_t mega_phase_units(int type, uint32_t n, uint32_t k, uint32_t segs, uint32_t D, uint32_t F, uint32_t &g_out, uint32_t most) {
     uint32_t g = pow2_floor_d(MG_STAGE_BYTES / (k * 2u * segs));
-    if (g * segs > 4) g = 4 / segs;
+    if (g * segs > most) g = most / segs;
     uint32_t units;
     if (type == 0 /* PH_QKV */) {
         while (g > 1 && (D / 2) % g != 0) g >>= 1;
@@ -132,12 +140,12 @@ __host__ __device__ inline uint32_t mega_phase_units(int type, uint32_t n, uint3
     return units;
 }
 // Phase p of the step: 5 per layer, then the LM head.  `T` = attention tiles over the cached tokens [0, pos).
-__device__ inline Phase phase_of(const MegaArgs &a, uint32_t p, uint32_t T) {
+template<bool NARROW> __device__ inline Phase phase_of(const MegaArgs &a, uint32_t p, uint32_t T) {
     Phase ph;
     ph.layer = p / 5;
     ph.type = ph.layer < a.layers ? static_cast<int>(p % 5) : PH_LM;
     ph.W = nullptr;
-    ph.n = ph.k = ph.g = ph.segs = ph.units = 0;
+    ph.n = ph.k = ph.g = ph.segs = ph.units = 0, ph.ng = 1;
     if (ph.type == PH_ATT) return ph;// attention units are assigned by att_range, not by unit_range
     const MegaLayer &L = a.layer[ph.layer < a.layers ? ph.layer : 0];
     switch (ph.type) {
@@ -147,7 +155,8 @@ __device__ inline Phase phase_of(const MegaArgs &a, uint32_t p, uint32_t T) {
         case PH_DOWN: ph.W = static_cast<const uint8_t *>(L.wd), ph.n = a.H, ph.k = a.F, ph.segs = 1; break;
         default: ph.W = static_cast<const uint8_t *>(a.lm_head), ph.n = a.V, ph.k = a.H, ph.segs = 1; break;
     }
-    ph.units = mega_phase_units(ph.type, ph.n, ph.k, ph.segs, a.D, a.F, ph.g);
+    ph.units = mega_phase_units(ph.type, ph.n, ph.k, ph.segs, a.D, a.F, ph.g, !NARROW || ph.type == PH_O ? 4 : 4 * mega_groups(ph.k));// O: every group would merge all the attention records
+    ph.ng = NARROW && ph.g * ph.segs > 4 ? ph.g * ph.segs / 4 : 1;// powers of two all
     return ph;
 }
 // first row of segment s of unit u and how many of its g rows exist
@@ -187,9 +196,9 @@ struct MegaCursor {
     bool done;
 };
 // Moves to the first phase >= c.p in which this CTA has units.
-__device__ inline void mega_cursor_seek(const MegaArgs &a, MegaCursor &c, uint32_t nphases, uint32_t NT) {
+template<bool NARROW> __device__ inline void mega_cursor_seek(const MegaArgs &a, MegaCursor &c, uint32_t nphases, uint32_t NT) {
     for (; c.p < nphases; ++c.p) {
-        c.ph = phase_of(a, c.p, NT);
+        c.ph = phase_of<NARROW>(a, c.p, NT);
         uint32_t u0;
         c.head = 0;
         if (c.ph.type == PH_ATT) {
@@ -202,10 +211,10 @@ __device__ inline void mega_cursor_seek(const MegaArgs &a, MegaCursor &c, uint32
     }
     c.done = true;
 }
-__device__ __forceinline__ void mega_cursor_advance(const MegaArgs &a, MegaCursor &c, uint32_t nphases, uint32_t NT) {
+template<bool NARROW> __device__ __forceinline__ void mega_cursor_advance(const MegaArgs &a, MegaCursor &c, uint32_t nphases, uint32_t NT) {
     if (++c.u >= c.u1) {
         ++c.p;
-        mega_cursor_seek(a, c, nphases, NT);
+        mega_cursor_seek<NARROW>(a, c, nphases, NT);
     }
 }
 // The (up to two) contiguous pieces of the cursor's unit: returns the piece count, fills source, bytes and ring offset.
@@ -293,7 +302,40 @@ __device__ __forceinline__ bool mega_linear_units(const uint8_t *smem, uint64_t 
     return true;
 }
 
-template<class T>
+// The same for narrow layers: NG groups of 256 / NG threads, group q taking rows 4 q .. 4 q + 3 of a unit of 4 NG rows, a thread one
+// chunk of each.  With four rows a unit and half or more of the threads without a chunk, the LM head of a 1024-wide model
+// (65 MB) took 25.9 us and takes 12.2 now, the whole 8-layer step 315 us and 291.
+template<class T, int NG>
+__device__ __forceinline__ bool mega_linear_units_narrow(const uint8_t *smem, uint64_t *full, uint64_t *empty, float *part, const float (&x)[8], uint32_t nu,
+                                                         uint32_t &it, uint32_t k, uint32_t tid, uint32_t warp, uint32_t lane) {
+    constexpr uint32_t GT = MG_CONSUMERS / NG, GW = MG_NW / NG;
+    const uint32_t row_bytes = k * 2u, group = tid / GT, sub = tid % GT;
+    const bool live = sub < k / 8;
+    for (uint32_t i = 0; i < nu; ++i, ++it) {
+        const uint32_t s = it % MG_STAGES, par = (it / MG_STAGES) & 1u;
+        if (!mbar_wait(&full[s], par)) return false;
+        const uint8_t *st = smem + s * MG_STAGE_BYTES + group * 4 * row_bytes + sub * 16;
+        uint4 raw[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) raw[r] = live ? *reinterpret_cast<const uint4 *>(st + r * row_bytes) : make_uint4(0, 0, 0, 0);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float w[8];
+            unpack8<T>(raw[r], w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[r] = fmaf(w[j], x[j], acc[r]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+        mg_reduce_halving<4>(acc, static_cast<int>(lane));
+        if ((lane & 7u) == 0) part[i * (4 * MG_NW) + (group * 4 + (lane >> 3)) * GW + warp % GW] = acc[0];
+    }
+    return true;
+}
+
+// NARROW: some rows have at most 1024 columns (the group count is then looked up per phase)
+template<class T, bool NARROW>
 __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + MG_STAGES * MG_STAGE_BYTES);
@@ -335,7 +377,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
         if (lane == 0) {
             const uint64_t policy = l2_policy_evict_first();
             MegaCursor ld{0, 0, 0, 0, {}, false};
-            mega_cursor_seek(a, ld, nphases, NT);
+            mega_cursor_seek<NARROW>(a, ld, nphases, NT);
             for (uint32_t it = 0; !ld.done; ++it) {
                 const uint32_t s = it % MG_STAGES, par = (it / MG_STAGES) & 1u;
                 if (!mbar_wait(&empty[s], par ^ 1u)) {
@@ -352,7 +394,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                     else
                         bulk_g2s_hint(st + dst[i], src[i], bytes[i], &full[s], policy);
                 }
-                mega_cursor_advance(a, ld, nphases, NT);
+                mega_cursor_advance<NARROW>(a, ld, nphases, NT);
             }
         }
         return;
@@ -374,11 +416,13 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
     auto prework = [&](uint32_t pn) {
         const uint32_t layer = pn / 5;
         const int type = layer < a.layers ? static_cast<int>(pn % 5) : PH_LM;
+        uint32_t first = tid;// this thread's first chunk (narrow: its only one)
+        if constexpr (NARROW) first = tid % (MG_CONSUMERS / phase_of<NARROW>(a, pn, NT).ng);
         if (type == PH_QKV || type == PH_GU || type == PH_LM) {
             const T *gamma = static_cast<const T *>(type == PH_LM ? a.norm_f : type == PH_QKV ? a.layer[layer].norm1 : a.layer[layer].norm2);
 #pragma unroll
             for (int c = 0; c < MG_KCH; ++c) {
-                const uint32_t ci = tid + c * MG_CONSUMERS;
+                const uint32_t ci = first + c * MG_CONSUMERS;
                 pre[c] = ci < a.H / 8 ? __ldg(reinterpret_cast<const uint4 *>(gamma + ci * 8)) : make_uint4(0, 0, 0, 0);
             }
         } else if (type == PH_O) {
@@ -386,7 +430,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
             const uint32_t kvrep = a.nH / a.nKV;
 #pragma unroll
             for (int c = 0; c < MG_KCH; ++c) {
-                const uint32_t ci = tid + c * MG_CONSUMERS;
+                const uint32_t ci = first + c * MG_CONSUMERS;
                 pre[c] = make_uint4(0, 0, 0, 0);
                 if (ci < a.nH * a.D / 8) {
                     const uint32_t h = ci * 8 / a.D, d0 = ci * 8 % a.D;
@@ -451,7 +495,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
     prework(0);
 
     for (uint32_t p = 0; p < nphases && ok; ++p) {
-        const Phase ph = phase_of(a, p, NT);
+        const Phase ph = phase_of<NARROW>(a, p, NT);
         uint32_t u0, u1, att_head = 0;
         if (ph.type == PH_ATT) {
             if (!att_range(a, NT, blockIdx.x, G, att_head, u0, u1)) u0 = u1 = 0;
@@ -596,6 +640,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
 
         // ---------------- linear phases ----------------
         const uint32_t kchunks = ph.k / 8;
+        const uint32_t first = NARROW ? tid % (MG_CONSUMERS / ph.ng) : tid;
         float x[MG_KCH][8];
         {
             // activation vector of this phase, in registers
@@ -619,7 +664,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                 const uint32_t splits = att_splits(G, a.nH);
 #pragma unroll
                 for (int c = 0; c < MG_KCH; ++c) {
-                    const uint32_t ci = tid + c * MG_CONSUMERS;
+                    const uint32_t ci = first + c * MG_CONSUMERS;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) x[c][j] = 0.f;
                     if (ci < kchunks) {
@@ -675,7 +720,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                 float ss = 0.f;
 #pragma unroll
                 for (int c = 0; c < MG_KCH; ++c) {
-                    const uint32_t ci = tid + c * MG_CONSUMERS;
+                    const uint32_t ci = first + c * MG_CONSUMERS;
                     if (ci < kchunks) {
                         unpack8<T>(__ldcg(reinterpret_cast<const uint4 *>(src + ci * 8)), x[c]);
                     } else {
@@ -691,12 +736,13 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                     mg_consumer_bar();
                     float tot = 0.f;
 #pragma unroll
-                    for (int w = 0; w < MG_NW; ++w) tot += red[w];
+                    for (int w = 0; w < MG_NW; ++w)
+                        if (!NARROW || w < static_cast<int>(MG_NW / ph.ng)) tot += red[w];// every group holds the whole vector
                     mg_consumer_bar();
                     const float rstd = rsqrtf(tot / static_cast<float>(ph.k) + a.eps);
 #pragma unroll
                     for (int c = 0; c < MG_KCH; ++c) {
-                        const uint32_t ci = tid + c * MG_CONSUMERS;
+                        const uint32_t ci = first + c * MG_CONSUMERS;
                         if (ci < kchunks) {
                             float gw[8];
                             unpack8<T>(pre[c], gw);
@@ -714,7 +760,10 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
         // phase: dispatch once to a fully unrolled loop so that all shared-memory loads of a unit are in flight together
         const uint32_t kc_live = (kchunks + MG_CONSUMERS - 1) / MG_CONSUMERS;
 #define RG_MG_RUN(R_, KC_) ok = mega_linear_units<T, R_, KC_>(smem, full, empty, part, x, nu, it, ph.k, tid, warp, lane)
-        if (R == 4) {
+        if (NARROW && ph.ng == 2) ok = mega_linear_units_narrow<T, 2>(smem, full, empty, part, x[0], nu, it, ph.k, tid, warp, lane);
+        else if (NARROW && ph.ng == 4) ok = mega_linear_units_narrow<T, 4>(smem, full, empty, part, x[0], nu, it, ph.k, tid, warp, lane);
+        else if (NARROW && ph.ng == 8) ok = mega_linear_units_narrow<T, 8>(smem, full, empty, part, x[0], nu, it, ph.k, tid, warp, lane);
+        else if (R == 4) {
             if (kc_live <= 2) RG_MG_RUN(4, 2);
             else if (kc_live <= 4) RG_MG_RUN(4, 4);
             else RG_MG_RUN(4, 6);
@@ -743,10 +792,12 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                 const uint32_t r = e % g, lu = e / g, u = u0 + lu;
                 float val[2] = {0.f, 0.f};
                 for (uint32_t sg = 0; sg < ph.segs; ++sg) {
-                    const float *pp = part + ((lu * 4) + (sg * g + r)) * MG_NW;
+                    const uint32_t gw = NARROW ? MG_NW / ph.ng : MG_NW;// warps that hold a part of a row's sum
+                    const float *pp = part + lu * (4 * MG_NW) + (sg * g + r) * gw;
                     float t = 0.f;
 #pragma unroll
-                    for (int w = 0; w < MG_NW; ++w) t += pp[w];
+                    for (int w = 0; w < MG_NW; ++w)
+                        if (!NARROW || w < static_cast<int>(gw)) t += pp[w];
                     val[sg] = t;
                 }
                 uint32_t rows;
@@ -912,7 +963,7 @@ int rg_b200_decode_step(const rg_decode_step_params *p, void *ws, const void *co
                                        {PH_LM, p->vocab, H, 1}};
         for (auto const &sh : shapes) {
             uint32_t g = 0;
-            const uint32_t units = mega_phase_units(static_cast<int>(sh[0]), sh[1], sh[2], sh[3], D, F, g);
+            const uint32_t units = mega_phase_units(static_cast<int>(sh[0]), sh[1], sh[2], sh[3], D, F, g, 4);// the narrow layers' units are fewer
             if (g == 0 || (units + G - 1) / G > MG_PART_UNITS) return RG_ERR_SHAPE;
         }
     }
@@ -939,7 +990,9 @@ int rg_b200_decode_step(const rg_decode_step_params *p, void *ws, const void *co
     a.max_seq = p->max_seq;
     a.eps = p->epsilon, a.log2_theta = log2f(p->theta), a.scale = 1.0f / sqrtf(static_cast<float>(p->head_dim));
     const size_t smem = mega_smem_bytes();
-    void *kern = p->dtype == RG_FP16 ? reinterpret_cast<void *>(decode_mega_kernel<__half>) : reinterpret_cast<void *>(decode_mega_kernel<__nv_bfloat16>);
+    const bool narrow = mega_groups(p->hidden) > 1 || mega_groups(p->ffn) > 1;
+    void *kern = p->dtype == RG_FP16 ? (narrow ? reinterpret_cast<void *>(decode_mega_kernel<__half, true>) : reinterpret_cast<void *>(decode_mega_kernel<__half, false>))
+                                     : (narrow ? reinterpret_cast<void *>(decode_mega_kernel<__nv_bfloat16, true>) : reinterpret_cast<void *>(decode_mega_kernel<__nv_bfloat16, false>));
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     // cooperative launch: all CTAs are resident together, which the grid barriers rely on
     void *args[] = {&a};
