@@ -20,9 +20,13 @@ int gemm_tc_qkv_rope(const rg_linear_params *p, const void *const *in, void *con
 int gemm_tc_push(const rg_mat_mul_params *p, const void *const *in, const ArPeers &peers, cudaStream_t st);
 bool gemm_tc_supported(const rg_mat_mul_params *p, const void *const *in, void *const *out);
 // fp32 product on the tensor cores, three bf16 parts per operand (gemm_tc32.cu); trans_a = 0
-bool gemm_tc32_preferred(const rg_mat_mul_params *p);
+float gemm_tc32_us(const rg_mat_mul_params *p);// estimated time
 size_t gemm_tc32_workspace(const rg_mat_mul_params *p);// split-K partials and arrival counters (zero before first use)
 int gemm_tc32(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st);
+// fp32 product on CUDA cores, 32 x 32 tiles with k divided over the warps (gemm_small32.cu); trans_a = 0
+bool gemm_small32_supported(const rg_mat_mul_params *p);
+float gemm_small32_us(const rg_mat_mul_params *p);
+int gemm_small32(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st);
 // Weight-streaming linear layer for 5..32 rows of X on the warp-level tensor path (linear_skinny.cu).
 struct SkinnyCall {
     int dtype;

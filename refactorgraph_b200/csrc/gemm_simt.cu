@@ -1,7 +1,6 @@
 // General MatMul on CUDA cores: any transpose combination, batch strides with broadcast, bias, alpha/beta,
 // fp32 accumulation.  This is the catch-all behind rg_b200_mat_mul (MatMulInfo semantics,
-// src/04kernel/src/attributes/mat_mul_info.cc:27-42); the decoder's large and skinny GEMMs are routed to the
-// tcgen05 and streaming kernels instead.
+// src/04kernel/src/attributes/mat_mul_info.cc:27-42) and takes what the tcgen05, streaming and 32 x 32 fp32 kernels do not.
 #include "common.cuh"
 #include "gemm_dispatch.cuh"
 

@@ -409,9 +409,13 @@ static Tc32Plan tc32_plan(const rg_mat_mul_params *p) {
     pl.partial_bytes = pl.splits > 1 ? static_cast<size_t>(pl.tiles) * pl.splits * T3_BM * pl.bn * 4 : 0;
     return pl;
 }
-bool gemm_tc32_preferred(const rg_mat_mul_params *p) {
-    if (p->dtype != RG_F32 || p->trans_a || p->k < 32) return false;
-    return static_cast<uint64_t>(p->m) * p->n * p->k * p->batch >= (1ull << 20);
+// 8 us before the first result, then the longest chain of k-blocks on an SM at 2 us (128 columns) or 1.3 us, and the parked sums
+float gemm_tc32_us(const rg_mat_mul_params *p) {
+    const Tc32Plan pl = tc32_plan(p);
+    const uint32_t sms = static_cast<uint32_t>(sm_count()), kblocks = (p->k + T3_BK - 1) / T3_BK;
+    const uint64_t rounds = (static_cast<uint64_t>(pl.tiles) * pl.splits + sms - 1) / sms;
+    return 8.f + static_cast<float>(rounds) * static_cast<float>((kblocks + pl.splits - 1) / pl.splits) * (pl.bn == 128 ? 2.0f : 1.3f) +
+           (pl.splits > 1 ? 2.f + 0.6f * static_cast<float>(pl.splits) : 0.f);
 }
 size_t gemm_tc32_workspace(const rg_mat_mul_params *p) {
     const Tc32Plan pl = tc32_plan(p);

@@ -58,12 +58,20 @@ static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *i
     return linear_skinny(c, ws, lin, lout, st);
 }
 
+// fp32 (force_kernel values): the form with the smaller estimated time.  Measured both ways (tensor cores / 32 x 32 tiles):
+// 32 x 256 x 256 9.0 / 4.1 us, 128 x 1024 x 1024 19.7 / 19.0, 256 x 1024 x 1024 20.1 / 19.3, 32 x 32000 x 1024 49 / 66, 4 x 11008 x 4096 75 / 103,
+// 509 x 2752 x 1024 39 / 91.
+static int f32_route(const rg_mat_mul_params *p) {
+    if (p->trans_a || !gemm_small32_supported(p)) return p->trans_a ? 1 : 5;
+    return gemm_tc32_us(p) < gemm_small32_us(p) ? 5 : 6;
+}
+
 extern "C" {
 
 size_t rg_b200_mat_mul_workspace(const rg_mat_mul_params *p) {
     // the fp32 tensor-core kernel's and the skinny kernel's k-split need scratch
     if (!p || p->m == 0 || p->n == 0 || p->k == 0 || p->batch == 0) return 0;
-    if (p->dtype == RG_F32) return gemm_tc32_preferred(p) || (p->force_kernel == 5 && !p->trans_a) ? gemm_tc32_workspace(p) : 0;
+    if (p->dtype == RG_F32) return f32_route(p) == 5 || (p->force_kernel == 5 && !p->trans_a) ? gemm_tc32_workspace(p) : 0;
     if ((p->dtype != RG_FP16 && p->dtype != RG_BF16) || p->trans_a) return 0;
     return skinny_shape(p) ? linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0) : 0;
 }
@@ -83,9 +91,13 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         case 3: return gemm_tc_supported(p, in, out) ? gemm_tc(p, in, out, st) : RG_ERR_UNSUPPORTED;
         case 4: return skinny_shape(p) ? run_skinny(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
         case 5: return gemm_tc32(p, ws, in, out, st);
+        case 6: return gemm_small32(p, in, out, st);
         default: return RG_ERR_UNSUPPORTED;
     }
-    if (p->dtype == RG_F32) return gemm_tc32_preferred(p) ? gemm_tc32(p, ws, in, out, st) : gemm_simt(p, in, out, st);
+    if (p->dtype == RG_F32) {
+        const int route = f32_route(p);
+        return route == 5 ? gemm_tc32(p, ws, in, out, st) : route == 6 ? gemm_small32(p, in, out, st) : gemm_simt(p, in, out, st);
+    }
     if (gemv_preferred(p) && aligned16(in[0]) && aligned16(in[1])) {
         const int rc = run_gemv(p, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;

@@ -326,7 +326,7 @@ template<class T> static int topk_chunks(const void *x, uint32_t n) {
     constexpr uint32_t N = 16 / sizeof(T);
     if (!aligned16(x) || n % N != 0 || n < 1024) return 0;
     const uint32_t per = (n / N + TOPK_REG_THREADS - 1) / TOPK_REG_THREADS;
-    return per <= 1 ? 1 : per <= 4 ? 4 : per <= 8 ? 8 : per <= 16 ? 16 : 0;
+    return per <= 4 ? 4 : per <= 8 ? 8 : per <= 16 ? 16 : 0;
 }
 struct TopkLaunch {
     int staged;
@@ -357,7 +357,6 @@ static int topk_launch(const rg_topk_params *p, const void *const *in, void *con
     auto idx = static_cast<int64_t *>(out[1]);
 #define RG_TOPK(CH) (p->softmax ? topk_go<T, true, CH>(p, x, out[0], idx, st) : topk_go<T, false, CH>(p, x, out[0], idx, st))
     switch (topk_chunks<T>(x, p->n)) {
-        case 1: return RG_TOPK(1);
         case 4: return RG_TOPK(4);
         case 8: return RG_TOPK(8);
         case 16: return RG_TOPK(16);
@@ -378,7 +377,6 @@ static int topk_sample_go(const rg_topk_sample_params *p, const void *const *in,
 template<class T>
 static int topk_sample_launch(const rg_topk_sample_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     switch (topk_chunks<T>(in[0], p->n)) {
-        case 1: return topk_sample_go<T, 1>(p, in, out, st);
         case 4: return topk_sample_go<T, 4>(p, in, out, st);
         case 8: return topk_sample_go<T, 8>(p, in, out, st);
         case 16: return topk_sample_go<T, 16>(p, in, out, st);
