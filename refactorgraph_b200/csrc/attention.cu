@@ -477,12 +477,14 @@ static int decode_launch(const rg_attn_decode_params *p, void *ws, const void *c
     a.tiles_per_split = pl.tiles_per_split, a.max_splits = pl.max_splits, a.max_len = p->max_len;
     a.kv = p->kv;
     a.scale = 1.0f / sqrtf(static_cast<float>(D));
-    // The tensor-path kernel pays for its larger prologue only when there is enough work to stream (batch-1 launches of
-    // ~1000 tiles measured 17.4 us against 15.5 us for the general kernel; batch 32 x 32 heads 203 us against 263 us).
+    // The tensor-path kernel pays for its larger prologue from 64 (sequence, head) rows or 8192 tiles on: batch-1 launches of ~1000 tiles
+    // measured 17.4 us against 15.5 us for the general kernel; 2 x 32 heads of 64 and 300 tokens 7.5 and 7.8 us, 16 x 8 heads of 100 to
+    // 2000 tokens 19.0 and 23.7, 3 x 32 heads of 200 to 1500 14.4 and 16.5, 8 x 32 heads of 300 to 1200 22.1 and 27.6, batch 32 x 32
+    // heads 203 and 263.
     static const int mma_env = std::getenv("RG_B200_ATTN_MMA") ? atoi(std::getenv("RG_B200_ATTN_MMA")) : -1;
     const uint64_t work_tiles = static_cast<uint64_t>(p->batch) * p->n_heads * ((p->max_len + AD_TILE - 1) / AD_TILE);
     const int stages = mma_env >= 2 ? mma_env : 2;// batch-32 launch: 203 / 235 / 385 us with 2 / 3 / 4 stages (3 / 2 / 1 CTAs per SM)
-    const bool mma = D == 128 && sizeof(T) == 2 && mma_env != 0 && (mma_env > 0 || work_tiles >= 8192);
+    const bool mma = D == 128 && sizeof(T) == 2 && mma_env != 0 && (mma_env > 0 || work_tiles >= 8192 || static_cast<uint64_t>(p->batch) * p->n_heads >= 64);
     const size_t smem = mma ? stages * 2 * AM_TILE_BYTES + 2 * stages * 8 + 4 * (128 + 2) * 4
                             : 4 * AD_TILE * D * 2 + 16 + (D + AD_TILE + (AD_THREADS / (D / 8)) * D) * 4;
     void (*kern)(const DecodeArgs) = attn_decode_kernel<T, D>;
