@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         }
     } else {
         // ---- epilogue warps 0..3: TMEM lanes [32*warp, 32*warp + 32) = tile rows ----
-        pdl_wait();// C, Y and the split-K workspace may still be in use by the previous kernel
+        pdl_wait();// C and Y may still be in use by the previous kernel
         T *Y = static_cast<T *>(a.Y);
         const T *C = static_cast<const T *>(a.C);
         const bool c_rowmajor = C && a.c_col_stride == 1 && (a.c_row_stride % 8) == 0;
@@ -1087,7 +1087,7 @@ int gemm_tc_qkv_rope(const rg_linear_params *p, const void *const *in, void *con
 // Y[m, n/2] = silu(X Wg^T) * (X Wu^T), W = [gate rows ; up rows] (rg_b200_linear, epilogue 2, more than 64 tokens): one B tile
 // pairs 128 gate rows with their 128 up rows, so both halves of an output column meet in one accumulator.
 // Up to 64 tokens: the weights go on the instruction's M side (a tile = 64 gate rows + their 64 up rows), the tokens on its N
-// side, with the k-split / stream-K plan of the plain skinny product; the up half of a tile hands its sums to the gate half.
+// side, k divided over clusters as for the plain skinny product; the up half of a tile hands its sums to the gate half.
 bool gemm_tc_swiglu_small_shape(const rg_linear_params *p) {
     return (p->dtype == RG_FP16 || p->dtype == RG_BF16) && p->epilogue == 2 && p->prologue == 0 && p->m > 4 && p->m <= 64 &&
            p->n % 128 == 0 && p->n >= 128 && p->k % 8 == 0 && p->k >= 64 && encode_fn() != nullptr;

@@ -1,5 +1,6 @@
 // rg_b200_mat_mul: routes a MatMul (MatMulInfo semantics, src/04kernel/src/attributes/mat_mul_info.cc:27-42)
-// to one of the three hand-written kernels.  No vendor GEMM is linked.
+// to one of the hand-written kernels (16 bits: streaming GEMV, skinny, tcgen05, CUDA cores; fp32: tcgen05, 32 x 32 tiles, CUDA cores).
+// No vendor GEMM is linked.
 #include "gemm_dispatch.cuh"
 #include <cstdlib>
 
