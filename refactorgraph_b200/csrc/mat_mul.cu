@@ -41,11 +41,10 @@ static bool skinny_shape(const rg_mat_mul_params *p) {
     if (p->has_bias && (p->bias_col_stride > 1)) return false;
     return linear_skinny_shape(p->dtype, p->m, p->n, p->k);
 }
-// The automatic choice: up to 16 rows of A against few rows of B with a long k — the shape where the tcgen05 kernel has too
-// few 128-row tiles and pays for a deep split (measured: 1280 x 8192 weights 13.0 us here, 18.3 us there; the other
-// products of a decoder layer are 15-40 % faster on tcgen05).
+// The automatic choice: up to 8 rows of A against few rows of B with a long k.  Here / on tcgen05 at 8 rows: 1280 x 8192 weights 10.3 / 10.4
+// us, 2560 x 8192 14.2 / 15.3, 512 x 8192 7.7 / 9.0; at 16 rows 11.3 / 10.6, 15.4 / 15.5 and 9.1 / 9.1; larger products are 15-40 % faster there.
 static bool skinny_preferred(const rg_mat_mul_params *p) {
-    return skinny_enabled() && skinny_shape(p) && p->m <= 16 && p->n <= 2560 && p->k >= 4096;
+    return skinny_enabled() && skinny_shape(p) && p->m <= 8 && p->n <= 2560 && p->k >= 4096;
 }
 static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
     SkinnyCall c = {};
