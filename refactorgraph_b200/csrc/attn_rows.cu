@@ -256,10 +256,18 @@ static RowsPlan rows_plan(const rg_attention_params *p, bool aligned = true) {
     pl.part_bytes = pl.splits > 1 ? ctas * pl.splits * pl.R * (p->head_dim + 2) * 4 : 0;
     return pl;
 }
+// The alignment of K and V may change from call to call and with it the number of row blocks: the counters have a place of their own
+// that holds those of either plan, so that no call parks sums where another one counts.
+struct RowsWorkspace {
+    size_t cnt_bytes, part_bytes;
+};
+static RowsWorkspace rows_workspace(const rg_attention_params *p) {
+    const RowsPlan pl = rows_plan(p), pu = rows_plan(p, false);
+    return {pl.cnt_bytes > pu.cnt_bytes ? pl.cnt_bytes : pu.cnt_bytes, pl.part_bytes > pu.part_bytes ? pl.part_bytes : pu.part_bytes};
+}
 size_t attn_rows_workspace(const rg_attention_params *p) {
-    const RowsPlan pl = rows_plan(p), pu = rows_plan(p, false);// whichever alignment the buffers turn out to have
-    const size_t b = pl.cnt_bytes + pl.part_bytes, u = pu.cnt_bytes + pu.part_bytes;
-    return b > u ? b : u;
+    const RowsWorkspace w = rows_workspace(p);
+    return w.cnt_bytes + w.part_bytes;
 }
 
 template<class T, int D>
@@ -292,7 +300,7 @@ int attn_rows(const rg_attention_params *p, void *ws, const void *q, const void 
     if (!ws) pl.splits = 1;
     RowsArgs a = {};
     a.q = q, a.k = k, a.v = v, a.o = o, a.past = past;
-    a.cnt = static_cast<unsigned *>(ws), a.part = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + pl.cnt_bytes);
+    a.cnt = static_cast<unsigned *>(ws), a.part = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + rows_workspace(p).cnt_bytes);
     a.S = p->seq_len, a.rows = pl.rows, a.row_blocks = pl.row_blocks, a.splits = pl.splits, a.kv_tokens = kv_tokens;
     a.scale = 1.0f / sqrtf(static_cast<float>(p->head_dim));
     const uint64_t ctas = static_cast<uint64_t>(pl.row_blocks) * pl.splits * p->n_kv_heads * p->batch;

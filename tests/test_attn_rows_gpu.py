@@ -57,6 +57,23 @@ def test_unaligned_caches_no_workspace_and_workspace_reuse(dtype):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_a_workspace_serves_aligned_and_unaligned_caches(dtype):
+    """One workspace for calls whose row blocks differ in number (4 query rows or 2 to a block on aligned caches, 1 on unaligned
+    ones): the sums that one call parks must not lie where the other counts arrivals.  Every row of the output is written."""
+    N, nH, nKV, S, D, past, cap = 4, 32, 8, 1, 128, 1037, 1100
+    q, k, v, kc, vc = _case(dtype, N, nH, nKV, S, D, past, cap)
+    p = capi.AttentionParams(ops.DT[dtype], N, nH, nKV, S, D, cap, 1)
+    ws = torch.zeros(capi.workspace("attention", p), dtype=torch.uint8, device="cuda")
+    pt, qd, knew, vnew = torch.tensor([past], device="cuda"), q.cuda(), k.cuda(), v.cuda()
+    for off in (0, 1, 0, 1, 1, 0):
+        kd, vd = (torch.zeros(c.numel() + off, dtype=dtype, device="cuda")[off:].copy_(c.flatten()) for c in (kc, vc))
+        o = torch.full_like(qd, float("nan"))
+        capi.call("attention", p, [t.data_ptr() for t in (qd, knew, vnew, pt, kd, vd)], [o.data_ptr(), kd.data_ptr(), vd.data_ptr()],
+                  ws=ws.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        _check(o, q, k, v, kc, vc, past)
+
+
 def test_infinite_values_reach_only_the_rows_that_see_them():
     q, k, v, kc, vc = _case(torch.float32, 1, 2, 2, 4, 64, 100, 200)
     vc[0, 0, 150:] = float("inf")    # past the sequence
