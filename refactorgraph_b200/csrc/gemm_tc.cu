@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         pdl_wait();// C and Y may still be in use by the previous kernel
         T *Y = static_cast<T *>(a.Y);
         const T *C = static_cast<const T *>(a.C);
-        const bool c_rowmajor = C && a.c_col_stride == 1 && (a.c_row_stride % 8) == 0;
+        const bool c_rowmajor = C && a.c_col_stride == 1 && (a.c_row_stride % 8) == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;// 16-byte loads
         if (S > 1) cluster_wait();
         // the all-reduce call this product feeds: its number stays put until the receiving kernel behind this one has run
         uint32_t ar_flag_v = 0;

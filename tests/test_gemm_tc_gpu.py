@@ -172,6 +172,33 @@ def test_skinny_stream_k(dtype, m, n, k, residual):
 
 
 @pytest.mark.parametrize("dtype", HALF)
+@pytest.mark.parametrize("trans_b", [True, False])
+@pytest.mark.parametrize("m,n,k", [(70, 256, 64), (333, 4096, 1024), (1100, 4104, 1032), (40, 1024, 512)])
+def test_addend_that_starts_off_a_16_byte_boundary(dtype, trans_b, m, n, k):
+    """C may start at any element (a bias row, a residual, the matrices of a batch at any distance): it is then read element by
+    element, in the plain epilogue, behind clusters and on CTA pairs.  Integer data, exact."""
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-2, 3, (k, n)).astype(np.float32)
+    ad, bd = ops.dev(a).to(dtype), ops.dev(b.T.copy() if trans_b else b).to(dtype)
+    prod = ad.float() @ (bd.float().T if trans_b else bd.float())
+    assert torch.equal(prod.cpu(), torch.from_numpy(a @ b))
+    for shape in ((n,), (m, n)):
+        for off in (1, 4, 8):
+            c = torch.randint(-2, 3, (int(np.prod(shape)) + off,), device="cuda").to(dtype)[off:].view(shape)
+            y = ops.mat_mul(ad, bd, c, trans_b=trans_b, beta=2.0, force=3)
+            assert _ok()
+            assert torch.equal(y, (prod + 2 * c.float()).to(dtype))
+    if not trans_b and m * n * k < 2 ** 26:
+        return  # a batch of small products with weights [k, n] is not tcgen05's
+    p = capi.MatMulParams()
+    p.dtype, p.m, p.n, p.k, p.trans_b, p.alpha, p.beta, p.batch = ops.DT[dtype], m, n, k, int(trans_b), 1.0, 1.0, 2
+    p.stride_y, p.has_bias, p.bias_row_stride, p.bias_col_stride, p.stride_c, p.force_kernel = m * n, 1, n, 1, m * n + 3, 3
+    c, y = torch.randint(-2, 3, (2 * (m * n + 3),), device="cuda").to(dtype), torch.empty(2, m, n, dtype=dtype, device="cuda")
+    capi.call("mat_mul", p, [ad.data_ptr(), bd.data_ptr(), c.data_ptr()], [y.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(y, (prod + c.view(2, -1)[:, :m * n].view(2, m, n).float()).to(dtype))
+
+
+@pytest.mark.parametrize("dtype", HALF)
 def test_prefill_sized_and_auto_route(dtype):
     torch.backends.cuda.matmul.allow_tf32 = False
     g = torch.Generator(device="cuda").manual_seed(0)
