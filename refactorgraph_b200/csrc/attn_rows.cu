@@ -129,11 +129,11 @@ __global__ void __launch_bounds__(AR_THREADS) attn_rows_kernel(const RowsArgs a)
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (key[u] < k1 && key[u] < see[r]) mn = fmaxf(mn, s[r][u]);
-            const float corr = m[r] == -INFINITY ? 0.f : expf(m[r] - mn);
+            const float corr = m[r] == -INFINITY ? 0.f : expf(m[r] - mn), base = mn == -INFINITY ? 0.f : mn;// only scores of -inf so far: weights of 0, not exp(inf - inf)
             l[r] *= corr;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                p[r][u] = key[u] < k1 && key[u] < see[r] ? expf(s[r][u] - mn) : 0.f;
+                p[r][u] = key[u] < k1 && key[u] < see[r] ? expf(s[r][u] - base) : 0.f;
                 l[r] += p[r][u];
             }
             m[r] = mn;

@@ -74,6 +74,21 @@ def test_a_workspace_serves_aligned_and_unaligned_caches(dtype):
         _check(o, q, k, v, kc, vc, past)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,nH,nKV,S,D,past", [(1, 1, 1, 1, 128, 300), (1, 8, 2, 1, 64, 1037), (1, 2, 2, 3, 32, 140), (1, 1, 1, 1, 256, 90)])
+@pytest.mark.parametrize("first", [0, 1])
+def test_keys_with_a_score_of_minus_infinity_have_no_weight(dtype, N, nH, nKV, S, D, past, first):
+    """Whole steps of a warp, whole splits and scattered keys whose scores are -inf, the leading key among them or not."""
+    cap = past + S + 7
+    q, k, v, kc, vc = _case(dtype, N, nH, nKV, S, D, past, cap)
+    q[..., 0] = q[..., 0].abs() + 0.5
+    for j in (*range(first, past // 2), *range(past // 2, past, 3)):
+        kc[:, :, j, 0] = float("-inf")
+    o = ops.attention(q.cuda(), k.cuda(), v.cuda(), past=past, k_cache=kc.cuda(), v_cache=vc.cuda())
+    assert bool(o.isfinite().all())
+    _check(o, q, k, v, kc, vc, past)
+
+
 def test_infinite_values_reach_only_the_rows_that_see_them():
     q, k, v, kc, vc = _case(torch.float32, 1, 2, 2, 4, 64, 100, 200)
     vc[0, 0, 150:] = float("inf")    # past the sequence
