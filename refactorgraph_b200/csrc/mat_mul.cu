@@ -13,9 +13,10 @@ static bool gemv_shape(const rg_mat_mul_params *p) {
 
 // The streaming kernel multiplies on the CUDA cores: one or two rows keep up with HBM (5.1-5.4 TB/s on large weights), three and four do
 // not (3.5), while the tensor cores pay about 3 us more per launch.  At four rows: 4096 x 4096 11.0 us here, 11.6 there; 12288 x
-// 4096 29.2 and 23.2; 22016 x 4096 50.9 and 36.5.  The line lies at 20 million weights.
-static bool gemv_preferred(const rg_mat_mul_params *p) {
-    return gemv_shape(p) && (p->m <= 2 || static_cast<uint64_t>(p->n) * p->k < 20000000ull);
+// 4096 29.2 and 23.2; 22016 x 4096 50.9 and 36.5.  The line lies at 20 million weights.  `tc`: the tensor cores take the product
+// (less than 64 x 64 results or an unaligned result they do not).
+static bool gemv_preferred(const rg_mat_mul_params *p, bool tc) {
+    return gemv_shape(p) && (p->m <= 2 || !tc || static_cast<uint64_t>(p->n) * p->k < 20000000ull);
 }
 
 static int run_gemv(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
@@ -43,8 +44,9 @@ static bool skinny_shape(const rg_mat_mul_params *p) {
 }
 // The automatic choice: up to 8 rows of A against few rows of B with a long k.  Here / on tcgen05 at 8 rows: 1280 x 8192 weights 10.3 / 10.4
 // us, 2560 x 8192 14.2 / 15.3, 512 x 8192 7.7 / 9.0; at 16 rows 11.3 / 10.6, 15.4 / 15.5 and 9.1 / 9.1; larger products are 15-40 % faster there.
-static bool skinny_preferred(const rg_mat_mul_params *p) {
-    return skinny_enabled() && skinny_shape(p) && p->m <= 8 && p->n <= 2560 && p->k >= 4096;
+// Up to 16 rows where tcgen05 does not take the product and the CUDA cores would be left with it.
+static bool skinny_preferred(const rg_mat_mul_params *p, bool tc) {
+    return skinny_enabled() && skinny_shape(p) && p->m <= (tc ? 8u : 16u) && p->n <= 2560 && p->k >= 4096;
 }
 static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *in, void *const *out, cudaStream_t st) {
     SkinnyCall c = {};
@@ -98,16 +100,16 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         const int route = f32_route(p);
         return route == 5 ? gemm_tc32(p, ws, in, out, st) : route == 6 ? gemm_small32(p, in, out, st) : gemm_simt(p, in, out, st);
     }
-    if (gemv_preferred(p) && aligned16(in[0]) && aligned16(in[1])) {
+    const bool tc = gemm_tc_supported(p, in, out);
+    if (gemv_preferred(p, tc) && aligned16(in[0]) && aligned16(in[1])) {
         const int rc = run_gemv(p, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;
     }
-    if (skinny_preferred(p) && aligned16(in[0]) && aligned16(in[1]) && aligned16(out[0]) &&
+    if (skinny_preferred(p, tc) && aligned16(in[0]) && aligned16(in[1]) && aligned16(out[0]) &&
         (ws || linear_skinny_workspace(p->dtype, p->m, p->n, p->k, p->has_bias ? 1 : 0, nullptr, 0) == 0)) {
         const int rc = run_skinny(p, ws, in, out, st);
         if (rc != RG_ERR_SHAPE && rc != RG_ERR_UNSUPPORTED) return rc;
     }
-    if (gemm_tc_supported(p, in, out)) return gemm_tc(p, in, out, st);
-    return gemm_simt(p, in, out, st);
+    return tc ? gemm_tc(p, in, out, st) : gemm_simt(p, in, out, st);
 }
 }

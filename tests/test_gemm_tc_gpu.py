@@ -199,6 +199,25 @@ def test_addend_that_starts_off_a_16_byte_boundary(dtype, trans_b, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", HALF)
+@pytest.mark.parametrize("m,n,k,force", [(4, 12288, 4096, 2), (9, 256, 8192, 4), (16, 128, 4096, 4), (8, 256, 8192, 4)])
+def test_the_automatic_route_of_products_too_small_for_tcgen05(dtype, m, n, k, force):
+    """Few rows against few weight rows (less than 64 x 64 results), or a result off a 16-byte boundary, are not left to the CUDA cores
+    where a streaming kernel takes them: the automatic route gives that kernel's bits."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, b = torch.randn(m, k, device="cuda", generator=g).to(dtype), torch.randn(n, k, device="cuda", generator=g).to(dtype)
+    want = ops.mat_mul(a, b, trans_b=True, force=force)
+    if m * n < 64 * 64:
+        assert torch.equal(ops.mat_mul(a, b, trans_b=True), want)
+    if force == 2:
+        p = capi.MatMulParams()
+        p.dtype, p.m, p.n, p.k, p.trans_b, p.alpha, p.beta, p.batch, p.stride_y = ops.DT[dtype], m, n, k, 1, 1.0, 1.0, 1, m * n
+        y = torch.empty(m * n + 1, dtype=dtype, device="cuda")[1:].view(m, n)
+        capi.call("mat_mul", p, [a.data_ptr(), b.data_ptr(), 0], [y.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(y, want)
+    assert _ok()
+
+
+@pytest.mark.parametrize("dtype", HALF)
 def test_prefill_sized_and_auto_route(dtype):
     torch.backends.cuda.matmul.allow_tf32 = False
     g = torch.Generator(device="cuda").manual_seed(0)
