@@ -264,9 +264,9 @@ def attention(q, k, v, past=None, k_cache=None, v_cache=None):
     pt = None if past is None else torch.tensor([past], dtype=torch.int64, device=q.device)
     nws = capi.workspace("attention", p)
     ws = torch.zeros(max(nws, 1), dtype=torch.uint8, device=q.device)
+    # the workspace goes back to the allocator on return, which hands it out again in the order of this stream
     capi.call("attention", p, [ptr(q), ptr(k), ptr(v), ptr(pt), ptr(k_cache), ptr(v_cache)],
               [ptr(o), ptr(k_cache), ptr(v_cache)], ws=ptr(ws) if nws else 0, stream=stream())
-    torch.cuda.current_stream().synchronize()  # the workspace is released on return
     return o
 
 

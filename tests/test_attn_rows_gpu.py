@@ -89,6 +89,21 @@ def test_keys_with_a_score_of_minus_infinity_have_no_weight(dtype, N, nH, nKV, S
     _check(o, q, k, v, kc, vc, past)
 
 
+def test_without_a_cache_it_can_be_captured():
+    q, k, v, _, _ = _case(torch.float32, 1, 4, 2, 6, 64, 0, 8)
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    want = ops.attention(q, k, v)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o = ops.attention(q, k, v)
+    o.fill_(float("nan"))
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(o, want)
+
+
 def test_infinite_values_reach_only_the_rows_that_see_them():
     q, k, v, kc, vc = _case(torch.float32, 1, 2, 2, 4, 64, 100, 200)
     vc[0, 0, 150:] = float("inf")    # past the sequence
