@@ -18,6 +18,7 @@
 #include "gemm_dispatch.cuh"
 #include "tcgen05.cuh"
 #include "ar_slots.cuh"
+#include <atomic>
 #include <cstdlib>
 #include <type_traits>
 #include <cuda.h>
@@ -925,16 +926,18 @@ static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs 
     // the whole shared-memory carve-out, so that a CTA of the next kernel can sit beside one of this kernel when both fit
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, static_cast<int>(cudaSharedmemCarveoutMaxShared)));
     const uint32_t tiles = ((a.n + BN - 1) / BN) * ((a.m + TC_BM - 1) / TC_BM), sms = static_cast<uint32_t>(sm_count());
-    static int clusters[64][4] = {};// per device and cluster size 1, 2, 4, 8; asked once
+    // per device and cluster size 1, 2, 4, 8; asked once (or by every thread that comes before the first answer, which is the same);
+    // the entry of size 1 says that the others are there
+    static std::atomic<int> clusters[64][4] = {};
     int dev = 0;
     RG_CHECK_CUDA(cudaGetDevice(&dev));
     int here[4] = {static_cast<int>(sms), 0, 0, 0};
     if (dev >= 0 && dev < 64) {
-        if (clusters[dev][0] == 0) {
-            for (int i = 3; i >= 1; --i) clusters[dev][i] = tc_resident_clusters(kern, 1u << i, smem);
-            clusters[dev][0] = static_cast<int>(sms);
+        if (clusters[dev][0].load(std::memory_order_acquire) == 0) {
+            for (int i = 3; i >= 1; --i) clusters[dev][i].store(tc_resident_clusters(kern, 1u << i, smem), std::memory_order_relaxed);
+            clusters[dev][0].store(static_cast<int>(sms), std::memory_order_release);
         }
-        for (int i = 0; i < 4; ++i) here[i] = clusters[dev][i];
+        for (int i = 0; i < 4; ++i) here[i] = clusters[dev][i].load(std::memory_order_relaxed);
     }
     const uint32_t kblocks = (a.k + TC_BK - 1) / TC_BK;
     if constexpr (BN <= 64) a.ksplit = tc_ksplit(tiles, kblocks, here);
@@ -967,14 +970,16 @@ static int tc_launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const Tc
     RG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const uint32_t items = ((a.n + BN - 1) / BN) * ((a.m + 2 * TC_BM - 1) / (2 * TC_BM));
     // as many pairs as the device can hold at once (asked once per device; half the SM count where the question fails)
-    static int resident[64] = {};
+    static std::atomic<int> resident[64] = {};
     int dev = 0;
     RG_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && resident[dev] == 0) {
+    int most = dev >= 0 && dev < 64 ? resident[dev].load(std::memory_order_relaxed) : sm_count() / 2;
+    if (most == 0) {
         const int n = tc_resident_clusters(kern, 2, smem);
-        resident[dev] = n > 0 ? n : sm_count() / 2;
+        most = n > 0 ? n : sm_count() / 2;
+        resident[dev].store(most, std::memory_order_relaxed);
     }
-    const uint32_t pairs = static_cast<uint32_t>(dev >= 0 && dev < 64 ? resident[dev] : sm_count() / 2);
+    const uint32_t pairs = static_cast<uint32_t>(most);
     const uint32_t grid = 2 * (items < pairs ? items : pairs);
     RG_CHECK_CUDA(launch_pdl_cluster(kern, dim3(grid), dim3(TC_THREADS), smem, st, 2u, ma, mb, a));
     count_launch();
