@@ -849,10 +849,6 @@ static bool tc_swapped(const rg_mat_mul_params *p) { return p->m <= 64 && p->n >
 // 1 / 2 / 4 / 8 CTAs: 4096 x 4096 21.4 / 13.6 / 11.7 / 14.3 us (model 22.8 / 13.1 / 10.1 / 14.4), 22016 x 4096 45.7 / 36.5 / 41.5 / 54.1 us,
 // 32000 x 1024 14.5 / 20.1 / 31.6 / 57.2 us, 57344 x 8192 174 / 156 / 151 / 193 us, 8192 x 28672 130 / 75 / 75 / 87 us.
 static uint32_t tc_ksplit(uint32_t tiles, uint32_t kblocks, const int (&clusters)[4]) {
-    if (const char *force = std::getenv("RG_B200_TC_KSPLIT")) {// tuning knob
-        const int f = std::atoi(force);
-        if ((f == 1 || f == 2 || f == 4 || f == 8) && static_cast<uint32_t>(f) <= kblocks && clusters[f == 1 ? 0 : f == 2 ? 1 : f == 4 ? 2 : 3] > 0) return static_cast<uint32_t>(f);
-    }
     const float sms = static_cast<float>(sm_count());
     uint32_t best = 1;
     float best_us = 1e30f;
