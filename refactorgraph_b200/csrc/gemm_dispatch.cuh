@@ -6,7 +6,8 @@ struct ArPeers;
 int gemm_simt(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st);
 int linear_stream(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
 // tcgen05/TMEM GEMM: Y[m,n] = alpha * A[m,k] * B[n,k]^T (+ beta*C), fp16/bf16, fp32 accumulation in TMEM.
-int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st);
+// pairs: on CTA pairs whatever the shape (RG_ERR_UNSUPPORTED where they are switched off)
+int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st, bool pairs = false);
 int gemm_tc_swiglu(const rg_linear_params *p, const void *const *in, void *const *out, cudaStream_t st);
 // SiLU gate on 5..64 tokens: weights on the instruction's M side, k split as for the skinny product
 bool gemm_tc_swiglu_small_shape(const rg_linear_params *p);

@@ -1008,7 +1008,8 @@ static int tc_wide_tile(uint32_t m, uint32_t n, uint32_t k) {
     return small < large ? TC_TILE_128 : TC_TILE_256;
 }
 
-int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
+int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st, bool pairs) {
+    if (pairs && !tc_pair_enabled()) return RG_ERR_UNSUPPORTED;
     const int is_bf16 = p->dtype == RG_BF16;
     const size_t es = 2;
     const bool mn = !p->trans_b;
@@ -1024,10 +1025,10 @@ int gemm_tc(const rg_mat_mul_params *p, const void *const *in, void *const *out,
         a.alpha = p->alpha, a.beta = p->beta, a.is_bf16 = is_bf16, a.k = p->k;
         CUtensorMap ma, mb;
         // a skinny activation matrix (m <= 64) goes on the N side of the instruction: D^T[n, m] = W[n,k] X[m,k]^T
-        const bool swap = tc_swapped(p);
+        const bool swap = !pairs && tc_swapped(p);
         uint32_t bn;
         if (!swap) {
-            const int tile = tc_wide_tile(p->m, p->n, p->k);
+            const int tile = pairs ? TC_TILE_PAIR : tc_wide_tile(p->m, p->n, p->k);
             bn = tile == TC_TILE_128 ? 128 : 256;
             a.m = p->m, a.n = p->n;
             a.early = (p->flags & RG_MM_B_STATIC) ? 2u : 0u;

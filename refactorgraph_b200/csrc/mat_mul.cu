@@ -94,6 +94,7 @@ int rg_b200_mat_mul(const rg_mat_mul_params *p, void *ws, const void *const *in,
         case 4: return skinny_shape(p) ? run_skinny(p, ws, in, out, st) : RG_ERR_UNSUPPORTED;
         case 5: return gemm_tc32(p, ws, in, out, st);
         case 6: return gemm_small32(p, in, out, st);
+        case 7: return gemm_tc_supported(p, in, out) ? gemm_tc(p, in, out, st, true) : RG_ERR_UNSUPPORTED;
         default: return RG_ERR_UNSUPPORTED;
     }
     if (p->dtype == RG_F32) {

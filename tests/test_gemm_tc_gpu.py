@@ -41,30 +41,32 @@ def test_against_numpy_oracle(dtype, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", HALF)
-@pytest.mark.parametrize("m,n,k", [(512, 256, 64), (1024, 768, 512), (600, 300, 200), (513, 1000, 4096), (2050, 256, 1032)])
-def test_pairs_of_ctas(dtype, m, n, k):
-    """512 rows and 256 columns or more: two CTAs share a 256 x 256 tile (tcgen05 ... cta_group::2), ragged edges included;
+@pytest.mark.parametrize("trans_b", [True, False])
+@pytest.mark.parametrize("m,n,k", [(512, 256, 64), (1024, 768, 512), (600, 300, 200), (513, 1000, 4096), (2050, 256, 1032), (1100, 4104, 1032)])
+def test_pairs_of_ctas(dtype, trans_b, m, n, k):
+    """Two CTAs share a 256 x 256 tile (tcgen05 ... cta_group::2; force_kernel = 7), ragged edges included, weights in either order;
     with a residual, alpha and beta; the second call must give the same bits."""
+    n = n if trans_b else (n + 7) // 8 * 8
     rng = np.random.default_rng(m * 7 + n + k)
     a = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(dtype)
-    b = torch.from_numpy((0.05 * rng.standard_normal((n, k))).astype(np.float32)).to(dtype)
+    b = torch.from_numpy((0.05 * rng.standard_normal((n, k) if trans_b else (k, n))).astype(np.float32)).to(dtype)
     c = torch.from_numpy(rng.standard_normal((m, n)).astype(np.float32)).to(dtype)
-    y = ops.mat_mul(a.cuda(), b.cuda(), trans_b=True, force=3)
+    y = ops.mat_mul(a.cuda(), b.cuda(), trans_b=trans_b, force=7)
     assert _ok()
-    want = onp.mat_mul(a.float().numpy(), b.float().numpy(), trans_b=True)
+    want = onp.mat_mul(a.float().numpy(), b.float().numpy(), trans_b=trans_b)
     np.testing.assert_allclose(y.float().cpu().numpy(), want, atol=2e-2, rtol=1e-2)
-    y2 = ops.mat_mul(a.cuda(), b.cuda(), c.cuda(), trans_b=True, alpha=0.5, beta=2.0, force=3)
+    y2 = ops.mat_mul(a.cuda(), b.cuda(), c.cuda(), trans_b=trans_b, alpha=0.5, beta=2.0, force=7)
     assert _ok()
-    want2 = onp.mat_mul(a.float().numpy(), b.float().numpy(), c.float().numpy(), trans_b=True, alpha=0.5, beta=2.0)
+    want2 = onp.mat_mul(a.float().numpy(), b.float().numpy(), c.float().numpy(), trans_b=trans_b, alpha=0.5, beta=2.0)
     np.testing.assert_allclose(y2.float().cpu().numpy(), want2, atol=4e-2, rtol=1e-2)
-    assert torch.equal(y, ops.mat_mul(a.cuda(), b.cuda(), trans_b=True, force=3))
+    assert torch.equal(y, ops.mat_mul(a.cuda(), b.cuda(), trans_b=trans_b, force=7))
 
 
 @pytest.mark.parametrize("dtype", HALF)
 @pytest.mark.parametrize("m,n,k", [(1, 4096, 512), (4, 1032, 64), (7, 1000, 1032), (33, 22016, 512), (64, 128, 72), (65, 64, 64), (100, 304, 72),
                                    (129, 136, 4096), (300, 4096, 1024), (511, 256, 200), (512, 264, 64), (700, 1000, 4096)])
 def test_weights_stored_k_by_n(dtype, m, n, k):
-    """trans_b = 0: the weights enter as an MN-major operand (on either side of the instruction, single CTAs and pairs).  Integer
+    """trans_b = 0: the weights enter as an MN-major operand (on either side of the instruction).  Integer
     data is exact in fp32 accumulation; the tolerance of the random data is the one of the K-major products."""
     rng = np.random.default_rng(m + 3 * n + k)
     a = rng.integers(-3, 4, (m, k)).astype(np.float32)
@@ -83,12 +85,12 @@ def test_weights_stored_k_by_n(dtype, m, n, k):
 
 @pytest.mark.parametrize("dtype", HALF)
 def test_pairs_of_ctas_bias_vector_and_batch(dtype):
-    """The pair kernel behind the batched call with a broadcast bias row (element-wise loads of C)."""
+    """The pair kernel behind the batched call with a broadcast bias row."""
     rng = np.random.default_rng(11)
     a = torch.from_numpy(rng.standard_normal((2, 520, 128)).astype(np.float32)).to(dtype)
     b = torch.from_numpy((0.1 * rng.standard_normal((2, 264, 128))).astype(np.float32)).to(dtype)
     c = torch.from_numpy(rng.standard_normal((264,)).astype(np.float32)).to(dtype)
-    y = ops.mat_mul(a.cuda(), b.cuda(), c.cuda(), trans_b=True, alpha=0.5, beta=2.0, force=3)
+    y = ops.mat_mul(a.cuda(), b.cuda(), c.cuda(), trans_b=True, alpha=0.5, beta=2.0, force=7)
     assert _ok()
     want = onp.mat_mul(a.float().numpy(), b.float().numpy(), c.float().numpy(), trans_b=True, alpha=0.5, beta=2.0)
     np.testing.assert_allclose(y.float().cpu().numpy(), want, atol=2e-2, rtol=1e-2)
@@ -151,10 +153,9 @@ def test_wide_clusters_share_a_tile(dtype, trans_b, m, n, k):
 
 @pytest.mark.parametrize("dtype", HALF)
 @pytest.mark.parametrize("m,n,k,residual", [(16, 22016, 4096, False), (32, 32000, 4096, True), (8, 20000, 4104, False)])
-def test_skinny_stream_k(dtype, m, n, k, residual):
-    """Skinny products with at least 64 k-blocks per SM run in stream-K mode: every CTA owns one contiguous run of
-    (tile, k-block) units and tiles that span CTAs are summed by the last to arrive.  The last case has a ragged last
-    row tile and a partial last k-block."""
+def test_skinny_products_of_several_tiles_a_cluster(dtype, m, n, k, residual):
+    """Skinny products with more tiles than clusters: the exchange of a tile's sums overlaps the stream of the next, the receive
+    buffers are used again.  The last case has a ragged last row tile and a partial last k-block."""
     rng = np.random.default_rng(m + n + k)
     a = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(dtype).cuda()
     b = torch.from_numpy((0.02 * rng.standard_normal((n, k))).astype(np.float32)).to(dtype).cuda()
