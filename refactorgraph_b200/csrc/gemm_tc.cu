@@ -653,22 +653,27 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             // 32 columns at a time.  What is added from C is fetched ahead of the accumulator (behind the stores of the columns before,
             // which may be the same memory as far as the compiler knows, every load would wait for its own round trip): one residual
             // tile of 128 x 256 took 12 us longer than the plain product with a load in front of every store.
-            const bool rows_wide = a.y_col_stride == 1 && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor);
+            // Rows of a multiple of 8 columns end between two 16-byte pieces, which are then there or not, and past the last column there is
+            // nothing to do: straight-line code for single columns costs more than its stores when it comes from a cold instruction cache
+            // (128 x 64 x 64 7.5 us with it, 1945 x 8040 x 312 33.4).
+            const bool rows_wide = a.y_col_stride == 1 && (a.n % 8) == 0 && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor);
             Vec16<T> cnext[4];
             auto fetch_c = [&](uint32_t col0) {
-                if (C && rows_wide && row < a.m && col0 + 32 <= a.n) {
+                if (C && rows_wide && row < a.m) {
                     const T *csrc = C + static_cast<uint64_t>(row) * a.c_row_stride + col0;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) cnext[j].load(csrc + 8 * j);
+                    for (int j = 0; j < 4; ++j)
+                        if (col0 + 8 * j < a.n) cnext[j].load(csrc + 8 * j);
                 }
             };
             auto store_columns = [&](const float (&r)[32], const Vec16<T> (&cv)[4], uint32_t col0) {
                 if (row >= a.m) return;
-                if (rows_wide && col0 + 32 <= a.n) {
+                if (rows_wide) {
                     // contiguous 64-byte run of this thread's row: four 16-byte stores
                     T *dst = Y + static_cast<uint64_t>(row) * a.y_row_stride + col0;
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
+                        if (col0 + j >= a.n) break;
                         float f[8];
 #pragma unroll
                         for (int e = 0; e < 8; ++e) f[e] = a.alpha * r[j + e];
@@ -684,10 +689,12 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     }
                 } else {
                     float add[32];
+                    if (C) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const uint32_t col = col0 + j;
-                        add[j] = C && col < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]) : 0.f;
+                        for (int j = 0; j < 32; ++j) {
+                            const uint32_t col = col0 + j;
+                            add[j] = col < a.n ? Num<T>::to_f(C[static_cast<uint64_t>(row) * a.c_row_stride + static_cast<uint64_t>(col) * a.c_col_stride]) : 0.f;
+                        }
                     }
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
@@ -749,6 +756,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             fetch_c(n0);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
+                if (n0 + c0 >= a.n) break;// the same for every thread
                 uint32_t r[32];
                 Vec16<T> cv[4];
 #pragma unroll
