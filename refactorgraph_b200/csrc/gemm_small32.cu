@@ -145,10 +145,11 @@ bool gemm_small32_supported(const rg_mat_mul_params *p) {
     const uint64_t tiles = static_cast<uint64_t>((p->m + S3_T - 1) / S3_T) * ((p->n + S3_T - 1) / S3_T);
     return p->dtype == RG_F32 && !p->trans_a && tiles <= 0x7fffffffull && p->batch <= 65535;
 }
-// Estimated time: launch and the last reduction 3 us, 12.5 ns per value of k for the first tile on an SM and 8.5 for each further one
+// Estimated time: launch and the last reduction 3 us, 12.5 ns per value of k for the first tile on an SM; each further one 0.85 us and 7.3 ns
+// per value of k
 float gemm_small32_us(const rg_mat_mul_params *p) {
     const uint64_t tiles = static_cast<uint64_t>((p->m + S3_T - 1) / S3_T) * ((p->n + S3_T - 1) / S3_T) * p->batch, sms = static_cast<uint64_t>(sm_count());
-    return 3.f + static_cast<float>(p->k) * (0.0125f + 0.0085f * static_cast<float>((tiles + sms - 1) / sms - 1));
+    return 3.f + 0.0125f * static_cast<float>(p->k) + static_cast<float>((tiles + sms - 1) / sms - 1) * (0.85f + 0.0073f * static_cast<float>(p->k));
 }
 int gemm_small32(const rg_mat_mul_params *p, const void *const *in, void *const *out, cudaStream_t st) {
     if (!gemm_small32_supported(p)) return RG_ERR_UNSUPPORTED;

@@ -60,12 +60,23 @@ static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *i
     return linear_skinny(c, ws, lin, lout, st);
 }
 
-// fp32 (force_kernel values): the form with the smaller estimated time.  Measured both ways (tensor cores / 32 x 32 tiles):
-// 32 x 256 x 256 9.0 / 4.1 us, 128 x 1024 x 1024 19.7 / 19.0, 256 x 1024 x 1024 20.1 / 19.3, 32 x 32000 x 1024 49 / 66, 4 x 11008 x 4096 75 / 103,
-// 509 x 2752 x 1024 39 / 91.
+// The 64 x 64 tiles of the CUDA-core kernel in fp32: a CTA alone takes 1.48 us for 16 values of k; with all SMs full a tile takes its SM 0.3 us
+// and 0.83 per 16 values
+static float f32_simt_us(const rg_mat_mul_params *p) {
+    const float tiles = static_cast<float>((p->m + 63) / 64) * static_cast<float>((p->n + 63) / 64) * static_cast<float>(p->batch);
+    const float steps = static_cast<float>((p->k + 15) / 16), alone = 1.48f * steps, full = tiles / static_cast<float>(sm_count()) * (0.3f + 0.83f * steps);
+    return 3.f + (alone > full ? alone : full);
+}
+// fp32 (force_kernel values): the form with the smallest estimated time.  Measured (tensor cores / 32 x 32 tiles / 64 x 64 tiles):
+// 32 x 256 x 256 9.0 / 4.1 / 18.2 us, 128 x 1024 x 1024 19.7 / 19.0 / 97.8, 256 x 1024 x 1024 20.1 / 19.3 / -, 32 x 32000 x 1024 49 / 66 / 295,
+// 4 x 11008 x 4096 75 / 103 / -, 509 x 2752 x 1024 39 / 91 / 128; the 64 x 64 tiles have the short k of large results, where the others pay
+// for every tile: 4096 x 4096 x 4 - / 111 / 34, 1024 x 1024 x 8 - / 8.5 / 3.9, 300 matrices of 100 x 100 x 10 - / 31 / 11, 512 of 64 x 64 x 64
+// - / 18.1 / 14.6.
 static int f32_route(const rg_mat_mul_params *p) {
     if (p->trans_a || !gemm_small32_supported(p)) return p->trans_a ? 1 : 5;
-    return gemm_tc32_us(p) < gemm_small32_us(p) ? 5 : 6;
+    const float tc = gemm_tc32_us(p), small = gemm_small32_us(p);
+    if ((p->m + 63) / 64 <= 65535 && f32_simt_us(p) < (tc < small ? tc : small)) return 1;
+    return tc < small ? 5 : 6;
 }
 
 extern "C" {
