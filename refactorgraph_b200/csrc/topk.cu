@@ -9,8 +9,9 @@
 //
 // In front of it, for rows of up to 16 16-byte chunks per thread: the row stays in registers (one read), every thread finds the
 // largest key of its own elements, and the k-th largest of those maxima is a key that at least k elements reach.  The elements that
-// reach it — k of them and a few more, unless values repeat a lot — are ranked against one another.  Only a row with more than 512
-// of them goes through the radix select, whose histogram passes serialise on the few distinct leading bytes that logits have:
+// reach it — k of them and a few more, unless values repeat a lot — are ranked against one another.  In a row with more than 512
+// of them, bisection finds the k-th largest key, and a pass in the order of the indices its first ties.
+// The histogram passes of the radix select serialise on the few distinct leading bytes that logits have:
 // one row of 32000 fp16 values 40 us, 509 rows of fp32 120 us, and a 4-token step of a two-layer decoder 527 -> 502 us without them.
 #include "common.cuh"
 
@@ -171,9 +172,84 @@ constexpr uint32_t TOPK_CAND = 512;
 struct TopkCand {
     uint32_t key[TOPK_CAND], idx[TOPK_CAND], count, top[32];
 };
-// The k winners of the row to sh.sort_key / sort_idx; false (for the whole block) when too many elements reach the threshold.
+// The sum of v over the block, for every thread; buf alternates between calls
+__device__ __forceinline__ uint32_t topk_block_count(uint32_t v, TopkCand &cd, uint32_t buf) {
+    const uint32_t lane = threadIdx.x & 31u, warps = blockDim.x >> 5;// at most 16
+    v = __reduce_add_sync(0xffffffffu, v);
+    if (lane == 0) cd.top[buf * 16 + (threadIdx.x >> 5)] = v;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, lane < warps ? cd.top[buf * 16 + lane] : 0u);
+}
+// The k winners to cd, of a row in which many keys reach `least`; `mine` is the largest key of the calling thread's elements.  A function of
+// its own that reads the row again (from L1 or L2), so that the common case has the registers to itself.  The k-th largest key by
+// bisection between `least` and the largest key (which are the same where those values repeat), then a pass in the order of the
+// indices that ends when enough ties are found.  A row of 32000 equal halves 47 us on the radix select.
+template<class T> static __device__ __noinline__ void topk_many_ties(const T *__restrict__ xr, uint32_t n, uint32_t k, uint32_t least, uint32_t mine, TopkCand &cd) {
+    constexpr uint32_t N = Vec16<T>::N;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, chunks = n / N;
+    mine = __reduce_max_sync(0xffffffffu, mine);
+    if (lane == 0) cd.top[16 + warp] = mine;
+    __syncthreads();// every thread has seen cd.count by now
+    if (threadIdx.x == 0) cd.count = 0;
+    // at least k keys reach lo, `above` (less than k) reach hi
+    uint32_t lo = least, hi = __reduce_max_sync(0xffffffffu, lane < warps ? cd.top[16 + lane] : 0u) + 1, above = 0, buf = 0;
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        uint32_t c = 0;
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < chunks; i += blockDim.x) {
+            Vec16<T> a;
+            float v[N];
+            a.load(xr + static_cast<size_t>(i) * N);
+            a.unpack(v);
+#pragma unroll
+            for (uint32_t j = 0; j < N; ++j) c += key_of<float>(v[j]) >= mid ? 1u : 0u;
+        }
+        c = topk_block_count(c, cd, buf);
+        buf ^= 1u;
+        if (c >= k) lo = mid;
+        else
+            hi = mid, above = c;
+    }
+    const uint32_t need = k - above;// ties, the first of them
+    uint32_t seen = 0;              // ties in the chunks before i0
+    for (uint32_t i0 = 0; i0 < chunks && (above || seen < need); i0 += blockDim.x, buf ^= 1u) {
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t key[N], ties = 0;
+        if (i < chunks) {
+            Vec16<T> a;
+            float v[N];
+            a.load(xr + static_cast<size_t>(i) * N);
+            a.unpack(v);
+#pragma unroll
+            for (uint32_t j = 0; j < N; ++j) key[j] = key_of<float>(v[j]), ties += key[j] == lo ? 1u : 0u;
+        }
+        uint32_t upto = ties;// of this warp's lanes so far
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, upto, d);
+            upto += lane >= d ? o : 0u;
+        }
+        if (lane == 31) cd.top[buf * 16 + warp] = upto;
+        __syncthreads();
+        const uint32_t w = lane < warps ? cd.top[buf * 16 + lane] : 0u;
+        uint32_t rank = seen + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + upto - ties;
+        seen += __reduce_add_sync(0xffffffffu, w);
+        if (i < chunks) {
+#pragma unroll
+            for (uint32_t j = 0; j < N; ++j) {
+                if (key[j] > lo || (key[j] == lo && rank++ < need)) {
+                    const uint32_t at = atomicAdd(&cd.count, 1u);// k of them in all
+                    cd.key[at] = key[j], cd.idx[at] = i * N + j;
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+// The k winners of the row to sh.sort_key / sort_idx
 template<class T, int CH>
-__device__ __forceinline__ bool topk_from_registers(const TopkRow<T, CH> &row, uint32_t k, TopkShared &sh, TopkCand &cd) {
+__device__ __forceinline__ void topk_from_registers(const TopkRow<T, CH> &row, const T *__restrict__ xr, uint32_t n, uint32_t k, TopkShared &sh, TopkCand &cd) {
     const uint32_t tid = threadIdx.x;
     uint32_t mine = 0u;
     row.each([&](float v, uint32_t) {
@@ -206,8 +282,11 @@ __device__ __forceinline__ bool topk_from_registers(const TopkRow<T, CH> &row, u
         });
     }
     __syncthreads();
-    const uint32_t count = cd.count;
-    if (count > TOPK_CAND) return false;
+    uint32_t count = cd.count;
+    if (count > TOPK_CAND) {
+        topk_many_ties<T>(xr, n, k, least, mine, cd);
+        count = cd.count;// k
+    }
     for (uint32_t c = tid; c < count; c += blockDim.x) {
         const uint32_t mk = cd.key[c], mi = cd.idx[c];
         uint32_t rank = 0;
@@ -215,7 +294,6 @@ __device__ __forceinline__ bool topk_from_registers(const TopkRow<T, CH> &row, u
         if (rank < k) sh.sort_key[rank] = mk, sh.sort_idx[rank] = mi;
     }
     __syncthreads();
-    return true;
 }
 
 // CH != 0: rows of CH chunks per thread, in registers
@@ -229,12 +307,12 @@ __global__ void __launch_bounds__(CH ? TOPK_REG_THREADS : TOPK_THREADS) topk_ker
     __shared__ TopkCand cd;
     const T *xr = x + static_cast<size_t>(blockIdx.x) * n;
     TopkRow<T, CH ? CH : 1> row;
-    bool done = false;
     if constexpr (CH != 0) {
         row.load(xr, n);
-        done = topk_from_registers(row, k, sh, cd);
+        topk_from_registers(row, xr, n, k, sh, cd);
+    } else {
+        topk_select<T>(xr, n, k, skeys, staged != 0, sh);
     }
-    if (!done) topk_select<T>(xr, n, k, skeys, staged != 0, sh);
     float inv_sum = 0.f, mx = 0.f;
     if constexpr (SOFTMAX) {
         mx = float_of_key(sh.sort_key[0]);
@@ -288,13 +366,13 @@ __global__ void __launch_bounds__(CH ? TOPK_REG_THREADS : TOPK_THREADS) topk_sam
     __shared__ TopkShared sh;
     __shared__ TopkCand cd;
     const T *xr = x + static_cast<size_t>(blockIdx.x) * n;
-    bool done = false;
     if constexpr (CH != 0) {
         TopkRow<T, CH> row;
         row.load(xr, n);
-        done = topk_from_registers(row, k, sh, cd);
+        topk_from_registers(row, xr, n, k, sh, cd);
+    } else {
+        topk_select<T>(xr, n, k, skeys, staged != 0, sh);
     }
-    if (!done) topk_select<T>(xr, n, k, skeys, staged != 0, sh);
     if (threadIdx.x == 0) {
         const float x0 = float_of_key(sh.sort_key[0]);
         float total = 0.f;
@@ -333,11 +411,10 @@ struct TopkLaunch {
     size_t smem;
     uint32_t threads;
 };
-// Keys are staged for the radix select; where it is only the way out of the register form and rows outnumber the SMs, staging would
-// halve the rows that run at a time and is left out
-static TopkLaunch topk_shape(uint32_t n, uint32_t rows, int ch) {
+// Keys are staged for the radix select
+static TopkLaunch topk_shape(uint32_t n, int ch) {
     TopkLaunch l;
-    l.staged = n <= TOPK_STAGE_MAX && (!ch || rows <= static_cast<uint32_t>(sm_count()));
+    l.staged = n <= TOPK_STAGE_MAX && !ch;
     l.smem = l.staged ? static_cast<size_t>(n) * 4 : 0;
     l.threads = ch ? static_cast<uint32_t>(TOPK_REG_THREADS) : topk_threads(n);
     return l;
@@ -345,7 +422,7 @@ static TopkLaunch topk_shape(uint32_t n, uint32_t rows, int ch) {
 
 template<class T, bool SOFTMAX, int CH>
 static int topk_go(const rg_topk_params *p, const T *x, void *values, int64_t *idx, cudaStream_t st) {
-    const TopkLaunch l = topk_shape(p->n, p->rows, CH);
+    const TopkLaunch l = topk_shape(p->n, CH);
     RG_CHECK_CUDA(cudaFuncSetAttribute(topk_kernel<T, SOFTMAX, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 163840));
     RG_CHECK_CUDA(launch_pdl(topk_kernel<T, SOFTMAX, CH>, dim3(p->rows), dim3(l.threads), l.smem, st, x, values, idx, p->n, p->k, l.staged));
     count_launch();
@@ -367,7 +444,7 @@ static int topk_launch(const rg_topk_params *p, const void *const *in, void *con
 
 template<class T, int CH>
 static int topk_sample_go(const rg_topk_sample_params *p, const void *const *in, void *const *out, cudaStream_t st) {
-    const TopkLaunch l = topk_shape(p->n, p->rows, CH);
+    const TopkLaunch l = topk_shape(p->n, CH);
     RG_CHECK_CUDA(cudaFuncSetAttribute(topk_sample_kernel<T, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 163840));
     RG_CHECK_CUDA(launch_pdl(topk_sample_kernel<T, CH>, dim3(p->rows), dim3(l.threads), l.smem, st, static_cast<const T *>(in[0]), static_cast<const uint64_t *>(in[1]),
                              static_cast<int64_t *>(out[0]), p->n, p->k, 1.0f / p->temperature, p->seed, l.staged));

@@ -605,7 +605,7 @@ def test_no_bounded_wait_expired():
 @pytest.mark.parametrize("dtype", [torch.float32] + HALF)
 @pytest.mark.parametrize("rows,n,k", [(1, 1024, 1), (3, 4096, 64), (2, 4104, 7), (2, 16384, 50), (1, 32768, 5), (2, 65536, 3), (150, 1031, 2)])
 def test_topk_rows_in_registers(rows, n, k, dtype):
-    """Row lengths on both sides of every register form; rows whose repeated values push them to the radix select; NaNs; an offset base."""
+    """Row lengths on both sides of every register form; rows whose repeated values go through the bisection; NaNs; an offset base."""
     rng = np.random.default_rng(n + k)
     x = rnd16(rng.standard_normal((rows, n)).astype(np.float32), dtype)
     x[0, ::3] = 2.0                      # more than 512 of them at or above the threshold
