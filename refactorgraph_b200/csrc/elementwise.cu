@@ -303,11 +303,16 @@ static int transpose_launch(const Idx4 &ix, const void *in, void *out, uint64_t 
     int j = -1;// the output axis that is innermost in the input
     for (int d = 0; d < 3; ++d)
         if (ix.shape[d] > 1 && ix.sa[d] == 1) j = d;
-    if (narrow && j >= 0 && ix.shape[3] >= 16 && ix.shape[j] >= 16) {
-        int o[2], n = 0;
-        for (int d = 0; d < 3; ++d)
+    // Tiles pay from about four million units on, where the strided side no longer lives in the caches, if they are nearly full: 16 x 16 x 509 x 64
+    // 29.6 us against 34.4 element by element, 4096 x 4096 51 and 67; 4 x 16 x 509 x 64 11.6 and 10.1, 64 x 64 x 16 x 16 13.5 and 4.4.
+    int o[2] = {0, 0};
+    uint64_t tiles = 0;
+    if (narrow && j >= 0 && total >= (1u << 22)) {
+        for (int d = 0, n = 0; d < 3; ++d)
             if (d != j) o[n++] = d;
-        const uint64_t tiles = static_cast<uint64_t>((ix.shape[3] + 31) / 32) * ((ix.shape[j] + 31) / 32) * ix.shape[o[0]] * ix.shape[o[1]];
+        tiles = static_cast<uint64_t>((ix.shape[3] + 31) / 32) * ((ix.shape[j] + 31) / 32) * ix.shape[o[0]] * ix.shape[o[1]];
+    }
+    if (tiles && tiles * 1024 * 4 <= total * 5) {
         const uint64_t cap = static_cast<uint64_t>(sm_count()) * 16;
         RG_CHECK_CUDA(launch_pdl(transpose_tile_kernel<U>, dim3(static_cast<unsigned>(tiles < cap ? tiles : cap)), dim3(256), 0, st, x, y, ix, j, o[0], o[1],
                                  static_cast<uint32_t>(tiles)));
