@@ -205,11 +205,13 @@ __global__ void softmax_row_kernel(const T *__restrict__ x, T *__restrict__ y, u
 // post == 1, rows of up to 8192 16-byte chunks (VEC) or single elements: the row lives in registers (CH chunks per thread), so it is read once and
 // every element costs one exponential: maximum, then exp and sum, then the scaled store.  (The online kernel above pays two
 // exponentials per element and reads the row twice: on [65536, 2048] fp16 it measured 289 us, issue-bound at 93 % SM throughput.)
-template<class T, int CH, bool VEC>
+// EARLY: launched so that the prologue overlaps the kernel before, which pays while all rows fit on the SMs at once; entering such a launch
+// costs every CTA (8144 rows of 512 halves: 8.8 us, 5.9 without; 32 rows of 32: 1.5 and 1.7).
+template<class T, int CH, bool VEC, bool EARLY>
 __global__ void __launch_bounds__(1024) softmax_row_reg_kernel(const T *__restrict__ x, T *__restrict__ y, uint32_t n) {
     constexpr int N = VEC ? Vec16<T>::N : 1;
     __shared__ float red[33];
-    pdl_enter();
+    if constexpr (EARLY) pdl_enter();
     const uint32_t chunks = n / N;
     const T *xr = x + static_cast<size_t>(blockIdx.x) * n;
     T *yr = y + static_cast<size_t>(blockIdx.x) * n;
@@ -293,9 +295,15 @@ static int softmax_launch(const rg_softmax_params *p, const void *const *in, voi
             ch = ch <= 1 ? 1 : ch <= 2 ? 2 : ch <= 4 ? 4 : 8;
             uint32_t t = ((work + ch - 1) / ch + 31) / 32 * 32;
             if (t < 32) t = 32;
-#define RG_SOFTMAX(CH) \
-    RG_CHECK_CUDA(vec ? launch_pdl(softmax_row_reg_kernel<T, CH, true>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid) \
-                      : launch_pdl(softmax_row_reg_kernel<T, CH, false>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid))
+            const uint64_t at_once = static_cast<uint64_t>(sm_count()) * (2048 / t < 32 ? 2048 / t : 32);
+#define RG_SOFTMAX(CH)                                                                                                                         \
+    if (p->pre <= at_once)                                                                                                                     \
+        RG_CHECK_CUDA(vec ? launch_pdl(softmax_row_reg_kernel<T, CH, true, true>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid)                  \
+                          : launch_pdl(softmax_row_reg_kernel<T, CH, false, true>, dim3(p->pre), dim3(t), 0, st, x, y, p->mid));               \
+    else if (vec)                                                                                                                              \
+        softmax_row_reg_kernel<T, CH, true, false><<<p->pre, t, 0, st>>>(x, y, p->mid);                                                        \
+    else                                                                                                                                       \
+        softmax_row_reg_kernel<T, CH, false, false><<<p->pre, t, 0, st>>>(x, y, p->mid)
             switch (ch) {
                 case 1: RG_SOFTMAX(1); break;
                 case 2: RG_SOFTMAX(2); break;
