@@ -622,8 +622,10 @@ def test_topk_rows_in_registers(rows, n, k, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.uint8, torch.float64])
 @pytest.mark.parametrize("shape,perm", [((7, 33, 65), (0, 2, 1)), ((2, 16, 31, 17), (0, 1, 3, 2)), ((3, 40, 2, 50), (3, 2, 1, 0)), ((1, 509, 4, 64), (0, 2, 1, 3)),
-                                        ((5, 6, 24), (1, 0, 2)), ((33, 1), (1, 0)), ((100, 200), (1, 0)), ((4, 3, 2, 15), (2, 0, 1, 3))])
+                                        ((5, 6, 24), (1, 0, 2)), ((33, 1), (1, 0)), ((100, 200), (1, 0)), ((4, 3, 2, 15), (2, 0, 1, 3)),
+                                        ((2, 1500, 1500), (0, 2, 1)), ((2, 1100, 2, 1040), (0, 3, 2, 1)), ((1040, 2, 3, 1100), (3, 1, 2, 0))])
 def test_transpose_tiles_and_wide_runs(shape, perm, dtype):
+    """Element by element, in runs of up to 16 bytes, and (four million units and more) in tiles."""
     x = (torch.arange(int(np.prod(shape))) % 251).reshape(shape).to(dtype).cuda()
     p = capi.TransposeParams()
     p.rank, p.elem_bytes = len(shape), x.element_size()
@@ -650,3 +652,16 @@ def test_binary_with_one_value_and_softmax_of_odd_rows(dtype):
         x[1, n // 2] = -np.inf if n > 1 else 0.0
         y = ops.softmax(ops.dev(x, dtype), 1)
         np.testing.assert_allclose(y.float().cpu().numpy(), onp.softmax_intended(x, 1), rtol=2e-5 if dtype == torch.float32 else 1e-2, atol=1e-9 if dtype == torch.float32 else 2e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32] + HALF)
+@pytest.mark.parametrize("rows,n", [(4736, 32), (4737, 32), (9000, 33), (2000, 1000), (700, 1023), (400, 4100)])
+def test_softmax_of_more_rows_than_fit_at_once(rows, n, dtype):
+    """Both sides of the line between an overlapped and an ordinary launch, in 16-byte pieces and in single elements; twice in a row, the
+    second on the results of the first."""
+    x = (3 * torch.randn(rows, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows + n))).to(dtype)
+    for _ in range(2):
+        y = ops.softmax(x, 1)
+        tol = dict(rtol=2e-5, atol=1e-9) if dtype == torch.float32 else dict(rtol=1e-2, atol=2e-3)
+        torch.testing.assert_close(y.double(), torch.softmax(x.double(), 1), **tol)
+        x = y
