@@ -2,13 +2,19 @@
 // (MatMulInfo semantics, src/04kernel/src/attributes/mat_mul_info.cc:27-42).  The CUDA cores bound the tiled kernel it stands in
 // for at 72 TFLOP/s; six bf16 products per fp32 product leave the tensor cores a bound of 265.
 //
-// Every operand x is written as hi + mid + lo, three bf16 values that together hold its 24 significand bits exactly: hi is x cut
-// (not rounded, so the largest finite values stay finite), mid the rounded rest, lo what is left.  Of the nine products of two
-// such sums the six largest are computed (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi); the other three are below 2^-24 of the
-// result.  The tensor core adds into fp32 but does not round to nearest, so the large product is not left to accumulate there:
-// its sum over 64 values of k goes to registers and is added with ordinary fp32 additions.  The five small products accumulate in
-// tensor memory over the whole k range, where their error is 2^-8 smaller.  Infinities and NaNs: they are in hi, so the sum of the
-// large product is already what fp32 gives; where it is not finite the small products (0 x inf, inf - inf) are left out.
+// Every operand x is written as hi + mid + lo, three bf16 values: hi is x rounded to eight significand bits, mid the rest rounded to eight,
+// lo what is left of it.  bf16 ends at 2^-133 and fp32 at 2^-149, so 2^16 x is what is taken apart: the three parts are then exactly
+// 2^16 x for every x below 2^112, subnormal numbers included, and the sums are 2^32 times as large until the last step.  Of the nine
+// products of two such sums the six largest are computed (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi); |mid| is at most 2^-8 |x| and
+// |lo| 2^-17 |x|, so the other three are together at most 2^-24 of the product of the values, as much as one rounding, with either sign.  The
+// tensor core adds into fp32 but does not round to nearest, so the large product is not left to accumulate there: its sum over 64
+// values of k goes to registers and is added with ordinary fp32 additions.  The five small products accumulate in tensor memory over
+// the whole k range, where their error is 2^-8 smaller.  Error against 64 bits (2-norm, normal data) here / of a chain of fp32
+// multiply-adds: k = 1 2.57e-8 / 2.52e-8, 2 2.6e-8 / 3.1e-8, 8 3.0e-8 / 5.3e-8, 64 0.69e-7 / 1.4e-7, 1024 0.91e-7 / 5.7e-7, 11008 1.3e-7 /
+// 1.9e-6; the automatic route leaves sums of fewer than eight products to the CUDA cores.  With all nine products but lo lo a single
+// product is as close as a multiply-add, and 509 x 32000 x 1024 takes 280 us.
+// Infinities, NaNs, operands from 2^112 and sums from 2^96 on leave a result that is not finite; such results are computed again
+// from the operands in fp32 multiply-adds, so they are what fp32 gives.
 //
 // D[i, j] = sum_k P[i, k] Q[j, k] on tiles of 128 x BN.  P = A and Q = B with BN = 128; up to 64 rows of A change sides, so that the
 // weights fill the 128 rows of the instruction and are converted once (BN = 32 or 64).  Either operand may be stored with k or with
@@ -21,10 +27,10 @@
 // FAST: rows on 16 bytes and k, and n where it is innermost, multiples of 8.  Addresses are then 32-bit offsets kept per item, rows past the
 // edge repeat the last one (they only reach results that are not stored) and only the last k-block looks at the end of k.  With
 // bounds and addresses worked out per piece the converters executed twice the instructions and set the pace: 509 x 2752 x 1024 45.3 us then,
-// 38.4 now; 509 x 32000 x 1024 281 and 235 (142 TFLOP/s); the prompt above 1.79 -> 1.61 ms
+// 38.4 without; 509 x 32000 x 1024 281 and 235.  The factor of 2^16 costs them 3 to 5 % where weights are stored [k, n] (41 and 249 us,
+// 134 TFLOP/s) and up to 10 % in the skinny forms.
 // k is split between CTAs where tiles are few; the last to arrive adds the parked sums in order.
-// Measured against the 64 x 64 CUDA-core tiles: a 509-token prompt through four layers of width 1024 with a 32000-word head
-// (86 GFLOP) 5.74 -> 2.06 ms, a 32-token prompt through two layers of width 256 446 -> 237 us.
+// Measured against the 64 x 64 CUDA-core tiles: 509 x 32000 x 1024 1433 us, 509 x 2752 x 1024 128, 32 x 32000 x 1024 295 (54 here).
 #include "gemm_dispatch.cuh"
 #include "tcgen05.cuh"
 
@@ -33,6 +39,7 @@ namespace rg {
 static __device__ int s_tc32_error;
 
 constexpr int T3_BM = 128, T3_BK = 64;
+constexpr float T3_SCALE = 65536.f, T3_UNSCALE = 1.f / (65536.f * 65536.f);// of the operands, and of the sums of their products
 
 template<int BN> struct Tc32Shape {
     static constexpr int STAGES = BN == 128 ? 2 : 3, GROUPS = BN == 32 ? 2 : 1, CONV = 8 * GROUPS, EPI = BN == 128 ? 8 : 4;
@@ -60,11 +67,6 @@ struct Tc32Args {
     float alpha, beta;
 };
 
-__device__ __forceinline__ uint32_t tc32_cut(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
 __device__ __forceinline__ uint32_t tc32_round(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -75,12 +77,12 @@ __device__ __forceinline__ void tc32_planes(const float (&v)[8], uint4 &hi, uint
     uint32_t w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const float a = v[2 * j], b = v[2 * j + 1];
-        const uint32_t h = tc32_cut(a, b);
+        const float a = v[2 * j] * T3_SCALE, b = v[2 * j + 1] * T3_SCALE;
+        const uint32_t h = tc32_round(a, b);
         const float a1 = a - __uint_as_float(h << 16), b1 = b - __uint_as_float(h & 0xffff0000u);
         const uint32_t m = tc32_round(a1, b1);
         const float a2 = a1 - __uint_as_float(m << 16), b2 = b1 - __uint_as_float(m & 0xffff0000u);
-        w[0][j] = h, w[1][j] = m, w[2][j] = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);// at most 8 bits are left: cutting is exact
+        w[0][j] = h, w[1][j] = m, w[2][j] = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);// at most 7 bits are left: cutting is exact
     }
     hi = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
     mid = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
@@ -115,6 +117,31 @@ struct Tc32Walk {
         return open(a, kblocks);
     }
 };
+
+// Results j0 + j of this lane's row i, j a bit of its `odd`, once more in fp32 multiply-adds: the parts of an infinity are not numbers, and the
+// scaled values and sums overflow where those of the operands do not.  The lanes share the k range of a result.  A function of its own
+// behind the stores of the others, so that it takes no registers from the converters' loop (inlined, 509 x 32000 x 1024 took 313 us
+// instead of 249).
+template<bool P_MN, bool Q_MN> static __device__ __noinline__ void tc32_mend(const Tc32Args &a, uint32_t b, uint32_t i, uint32_t j0, uint64_t odd) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t p_k = P_MN ? a.p.ld : 1, q_k = Q_MN ? a.q.ld : 1;
+    for (uint32_t l = 0; l < 32; ++l) {
+        const uint32_t row = __shfl_sync(0xffffffffu, i, l);
+        const float *p = a.p.x + b * a.p.stride + (P_MN ? row : static_cast<uint64_t>(row) * a.p.ld);
+        for (uint64_t left = __shfl_sync(0xffffffffu, odd, l); left; left &= left - 1) {
+            const uint32_t j = j0 + static_cast<uint32_t>(__ffsll(static_cast<long long>(left))) - 1;
+            const float *q = a.q.x + b * a.q.stride + (Q_MN ? j : static_cast<uint64_t>(j) * a.q.ld);
+            float s = 0.f;
+#pragma unroll 8
+            for (uint32_t k = lane; k < a.k; k += 32) s = fmaf(__ldg(p + k * p_k), __ldg(q + k * q_k), s);
+            s = warp_sum(s) * a.alpha;
+            if (lane == 0) {
+                if (a.C) s += a.beta * a.C[b * a.stride_c + row * a.c_i + j * a.c_j];
+                a.Y[b * a.stride_y + row * a.y_i + j * a.y_j] = s;
+            }
+        }
+    }
+}
 
 template<int BN, bool P_MN, bool Q_MN, bool FAST>
 __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(const __grid_constant__ Tc32Args a) {
@@ -319,8 +346,7 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
                 tmem_ld_32x16(tmem + (2 + (local & 1u)) * BN + col + c + lanes, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (fabsf(acc[c + j]) <= 3.402823466e38f) acc[c + j] += __uint_as_float(r[j]);
+                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
             }
             tc_fence_before();
             __syncwarp();
@@ -354,7 +380,18 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
                 }
                 if (threadIdx.x == 0) a.counter[tile] = 0u;
             }
+            uint64_t odd = 0;// results of this row that are not finite
             if (i < a.rows) {
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) acc[j] *= T3_UNSCALE;
+                float probe = 0.f;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) probe = fmaf(acc[j], 0.f, probe);
+                if (probe != 0.f) {
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j)
+                        if (!(fabsf(acc[j]) <= 3.402823466e38f) && j0 + j < a.cols) odd |= 1ull << j;
+                }
                 float *y = a.Y + b * a.stride_y + i * a.y_i + j0 * a.y_j;
 #pragma unroll
                 for (int j = 0; j < COLS; ++j) acc[j] *= a.alpha;
@@ -364,15 +401,16 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
                     for (int j = 0; j < COLS; ++j)
                         if (j0 + j < a.cols) acc[j] += a.beta * c[j * a.c_j];
                 }
-                if (a.y_j == 1 && j0 + COLS <= a.cols && (reinterpret_cast<uintptr_t>(y) & 15u) == 0) {
+                if (odd == 0 && a.y_j == 1 && j0 + COLS <= a.cols && (reinterpret_cast<uintptr_t>(y) & 15u) == 0) {
 #pragma unroll
                     for (int j = 0; j < COLS; j += 4) *reinterpret_cast<float4 *>(y + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
                 } else {
 #pragma unroll
                     for (int j = 0; j < COLS; ++j)
-                        if (j0 + j < a.cols) y[j * a.y_j] = acc[j];
+                        if (j0 + j < a.cols && (odd >> j & 1u) == 0) y[j * a.y_j] = acc[j];
                 }
             }
+            if (__any_sync(0xffffffffu, odd != 0)) tc32_mend<P_MN, Q_MN>(a, b, i, j0, odd);
         }
     }
     tc_fence_before();
@@ -409,12 +447,15 @@ static Tc32Plan tc32_plan(const rg_mat_mul_params *p) {
     pl.partial_bytes = pl.splits > 1 ? static_cast<size_t>(pl.tiles) * pl.splits * T3_BM * pl.bn * 4 : 0;
     return pl;
 }
-// 8 us before the first result, then the longest chain of k-blocks on an SM at 2 us (128 columns) or 1.3 us, and the parked sums
+// 8 us before the first result, then the longest chain of k-blocks on an SM at 1.8 us (128 columns), 1.45 or 1.4 us, 4.3 us (fewer columns: 1.2) for
+// every tile but the last on an SM (its results are stored while the next tile waits for the drainers), and the parked sums.  Rows off 16
+// bytes: 2.2 us a k-block, and 7 us a tile where it is the results' (16 x 509 x 509 x 64 28.5 us)
 float gemm_tc32_us(const rg_mat_mul_params *p) {
     const Tc32Plan pl = tc32_plan(p);
     const uint32_t sms = static_cast<uint32_t>(sm_count()), kblocks = (p->k + T3_BK - 1) / T3_BK;
     const uint64_t rounds = (static_cast<uint64_t>(pl.tiles) * pl.splits + sms - 1) / sms;
-    return 8.f + static_cast<float>(rounds) * static_cast<float>((kblocks + pl.splits - 1) / pl.splits) * (pl.bn == 128 ? 2.0f : 1.3f) +
+    return 8.f + static_cast<float>(rounds) * static_cast<float>((kblocks + pl.splits - 1) / pl.splits) * (pl.bn == 32 ? 1.4f : pl.bn == 64 ? 1.45f : p->k % 8 == 0 && (p->trans_b || p->n % 8 == 0) ? 1.8f : 2.2f) +
+           (pl.bn == 128 ? 4.3f : 1.2f) * static_cast<float>(rounds - 1) + (pl.bn == 128 && p->n % 4 ? 7.f * static_cast<float>(rounds) : 0.f) +
            (pl.splits > 1 ? 2.f + 0.6f * static_cast<float>(pl.splits) : 0.f);
 }
 size_t gemm_tc32_workspace(const rg_mat_mul_params *p) {

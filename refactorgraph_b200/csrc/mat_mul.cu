@@ -74,7 +74,7 @@ static float f32_simt_us(const rg_mat_mul_params *p) {
 // - / 18.1 / 14.6.
 static int f32_route(const rg_mat_mul_params *p) {
     if (p->trans_a || !gemm_small32_supported(p)) return p->trans_a ? 1 : 5;
-    const float tc = gemm_tc32_us(p), small = gemm_small32_us(p);
+    const float tc = p->k < 8 ? 1e30f : gemm_tc32_us(p), small = gemm_small32_us(p);
     if ((p->m + 63) / 64 <= 65535 && f32_simt_us(p) < (tc < small ? tc : small)) return 1;
     return tc < small ? 5 : 6;
 }

@@ -56,6 +56,70 @@ def test_shared_operand_of_a_batch_and_unaligned_operands(force):
         torch.testing.assert_close(ops.mat_mul(a, b, force=force).double(), a.double() @ b.double(), atol=3e-5, rtol=1e-5)
 
 
+@pytest.mark.parametrize("force", [0, 5, 6])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 8, 16, 24, 64, 100])
+def test_short_sums_are_as_close_as_fused_multiply_adds(force, trans_b, k):
+    """With few terms a product's own rounding is nearly all the error there is.  What the tensor-core form leaves out is at most 2^-24 of a
+    product and may show beside the one rounding of a sum of one (which the automatic route leaves to the CUDA cores); 2 % are for
+    the luck of the data."""
+    for m in (20, 64, 300):
+        g = torch.Generator(device="cuda").manual_seed(k + m)
+        a = torch.randn(m, k, device="cuda", generator=g)
+        b = torch.randn(*((1000, k) if trans_b else (k, 1000)), device="cuda", generator=g)
+        want = a.double() @ (b.double().T if trans_b else b.double())
+        simt, y = ops.mat_mul(a, b, trans_b=trans_b, force=1), ops.mat_mul(a, b, trans_b=trans_b, force=force)
+        assert _err(y, want) <= (1.06 if k == 1 and force == 5 else 1.02) * _err(simt, want)
+        if k == 1:
+            assert bool(((y.double() - want).abs() <= 2.0 ** -23 * want.abs()).all())
+
+
+@pytest.mark.parametrize("force", [5, 6])
+@pytest.mark.parametrize("m", [20, 60, 200])
+@pytest.mark.parametrize("k", [8, 300])
+@pytest.mark.parametrize("exponent", [-100, -110, -116, -120, -126, -133, -140, 120])
+def test_small_and_large_operands(force, m, k, exponent):
+    """One operand around 2^exponent (subnormal numbers from -126 down), the other the size that makes the result ordinary."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    for swap in (False, True):
+        scale = (2.0 ** (-exponent // 2), 2.0 ** exponent) if swap else (2.0 ** exponent, 2.0 ** (-exponent // 2))
+        a = (torch.rand(m, k, device="cuda", generator=g, dtype=torch.float64) * scale[0]).float()
+        b = (torch.rand(k, 132, device="cuda", generator=g, dtype=torch.float64) * scale[1]).float()
+        want = a.double() @ b.double()
+        simt, y = ops.mat_mul(a, b, force=1), ops.mat_mul(a, b, force=force)
+        assert _err(y, want) <= 1.02 * _err(simt, want)
+        assert bool(((y.double() - want).abs() <= (k + 16) * 2.0 ** -24 * want).all())
+
+
+@pytest.mark.parametrize("force", [5, 6])
+@pytest.mark.parametrize("m", [20, 60, 200])
+def test_results_that_are_subnormal(force, m):
+    """Products of 2^-140: no further off than a quantum (2^-149) a rounding, as a chain of fp32 multiply-adds."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b = (2.0 ** -70 * torch.randn(*s, device="cuda", generator=g) for s in ((m, 200), (200, 132)))
+    want = a.double() @ b.double()
+    simt, y = ops.mat_mul(a, b, force=1), ops.mat_mul(a, b, force=force)
+    assert _err(y, want) <= 1.02 * _err(simt, want)
+
+
+@pytest.mark.parametrize("force", [5, 6])
+@pytest.mark.parametrize("m", [20, 60, 200])
+def test_infinity_times_the_smallest_numbers(force, m):
+    """inf x 2^-149 is inf, inf x 0 is NaN, and sums that stay below the largest number stay finite."""
+    a, b = torch.ones(m, 72, device="cuda"), torch.ones(72, 140, device="cuda")
+    a[3, 70], a[m - 1, 5] = float("inf"), float("-inf")
+    b[70, 4], b[70, 5], b[5, 139] = 2.0 ** -149, 0.0, 2.0 ** -140
+    y, want = ops.mat_mul(a, b, force=force), ops.mat_mul(a, b, force=1)
+    assert want[3, 4] == float("inf") and want[3, 5].isnan() and want[m - 1, 139] == float("-inf")
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y[~y.isnan()], want[~want.isnan()])
+    a, b = torch.full((m, 2), 2.0 ** 63, device="cuda"), torch.full((2, 140), 2.0 ** 63 * (2 - 2.0 ** -10), device="cuda")
+    assert torch.equal(ops.mat_mul(a, b, force=force).double(), a.double() @ b.double())
+    a, b = torch.full((m, 1), 2.0 ** 64 * (1 - 2.0 ** -24), device="cuda"), torch.full((1, 140), 2.0 ** 64 * (1 - 2.0 ** -24), device="cuda")
+    assert torch.equal(ops.mat_mul(a, b, force=force).double(), torch.full((m, 140), 2.0 ** 128 * (1 - 2.0 ** -23), device="cuda", dtype=torch.float64))
+    c = torch.randn(m, 140, device="cuda")
+    assert torch.equal(ops.mat_mul(a, b, c, alpha=0.5, beta=2.0, force=force), ops.mat_mul(a, b, c, alpha=0.5, beta=2.0, force=1))
+
+
 @pytest.mark.parametrize("force", [5, 6])
 @pytest.mark.parametrize("m", [60, 200])
 def test_values_at_the_ends_of_the_range(force, m):
