@@ -118,27 +118,40 @@ struct Tc32Walk {
     }
 };
 
-// Results j0 + j of this lane's row i, j a bit of its `odd`, once more in fp32 multiply-adds: the parts of an infinity are not numbers, and the
-// scaled values and sums overflow where those of the operands do not.  The lanes share the k range of a result.  A function of its own
-// behind the stores of the others, so that it takes no registers from the converters' loop (inlined, 509 x 32000 x 1024 took 313 us
-// instead of 249).
-template<bool P_MN, bool Q_MN> static __device__ __noinline__ void tc32_mend(const Tc32Args &a, uint32_t b, uint32_t i, uint32_t j0, uint64_t odd) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t p_k = P_MN ? a.p.ld : 1, q_k = Q_MN ? a.q.ld : 1;
-    for (uint32_t l = 0; l < 32; ++l) {
-        const uint32_t row = __shfl_sync(0xffffffffu, i, l);
-        const float *p = a.p.x + b * a.p.stride + (P_MN ? row : static_cast<uint64_t>(row) * a.p.ld);
-        for (uint64_t left = __shfl_sync(0xffffffffu, odd, l); left; left &= left - 1) {
-            const uint32_t j = j0 + static_cast<uint32_t>(__ffsll(static_cast<long long>(left))) - 1;
-            const float *q = a.q.x + b * a.q.stride + (Q_MN ? j : static_cast<uint64_t>(j) * a.q.ld);
-            float s = 0.f;
-#pragma unroll 8
-            for (uint32_t k = lane; k < a.k; k += 32) s = fmaf(__ldg(p + k * p_k), __ldg(q + k * q_k), s);
-            s = warp_sum(s) * a.alpha;
-            if (lane == 0) {
-                if (a.C) s += a.beta * a.C[b * a.stride_c + row * a.c_i + j * a.c_j];
-                a.Y[b * a.stride_y + row * a.y_i + j * a.y_j] = s;
-            }
+// Results j0 + j of this lane's row i, j a bit of its `odd`, once more as chains of fp32 multiply-adds: the parts of an infinity are not
+// numbers, and the scaled values and sums overflow where those of the operands do not.  All lanes work on the columns that any of
+// them needs, eight at a time, so that a value of Q serves 32 rows and one of P eight columns.  A function of its own behind the
+// stores of the others, so that it takes no registers from the converters' loop (inlined, 509 x 32000 x 1024 took 313 us instead
+// of 249).
+template<int COLS, bool P_MN, bool Q_MN> static __device__ __noinline__ void tc32_mend(const Tc32Args &a, uint32_t b, uint32_t i, uint32_t j0, uint64_t odd) {
+    const uint64_t p_k = P_MN ? a.p.ld : 1, q_k = Q_MN ? a.q.ld : 1, q_j = Q_MN ? 1 : a.q.ld;
+    const uint32_t row = i < a.rows ? i : a.rows - 1;// a row past the edge repeats the last one and stores nothing
+    const float *p = a.p.x + b * a.p.stride + (P_MN ? row : static_cast<uint64_t>(row) * a.p.ld);
+    const uint64_t any = static_cast<uint64_t>(__reduce_or_sync(0xffffffffu, static_cast<uint32_t>(odd >> 32))) << 32 | __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(odd));
+    for (uint32_t g = 0; g < COLS; g += 8) {
+        if ((any >> g & 0xffu) == 0) continue;
+        const float *q = a.q.x + b * a.q.stride;
+        uint64_t at[8];
+        float s[8];
+#pragma unroll
+        for (uint32_t e = 0; e < 8; ++e) {
+            const uint32_t j = j0 + g + e;
+            at[e] = (j < a.cols ? j : a.cols - 1) * q_j, s[e] = 0.f;
+        }
+#pragma unroll 4
+        for (uint32_t k = 0; k < a.k; ++k, p += p_k, q += q_k) {
+            const float x = __ldg(p);
+#pragma unroll
+            for (uint32_t e = 0; e < 8; ++e) s[e] = fmaf(x, __ldg(q + at[e]), s[e]);
+        }
+        p -= a.k * p_k;
+#pragma unroll
+        for (uint32_t e = 0; e < 8; ++e) {
+            const uint32_t j = j0 + g + e;
+            if ((odd >> (g + e) & 1u) == 0) continue;
+            float y = s[e] * a.alpha;
+            if (a.C) y += a.beta * a.C[b * a.stride_c + row * a.c_i + j * a.c_j];
+            a.Y[b * a.stride_y + row * a.y_i + j * a.y_j] = y;
         }
     }
 }
@@ -410,7 +423,7 @@ __global__ void __launch_bounds__(Tc32Shape<BN>::THREADS, 1) gemm_tc32_kernel(co
                         if (j0 + j < a.cols && (odd >> j & 1u) == 0) y[j * a.y_j] = acc[j];
                 }
             }
-            if (__any_sync(0xffffffffu, odd != 0)) tc32_mend<P_MN, Q_MN>(a, b, i, j0, odd);
+            if (__any_sync(0xffffffffu, odd != 0)) tc32_mend<COLS, P_MN, Q_MN>(a, b, i, j0, odd);
         }
     }
     tc_fence_before();
