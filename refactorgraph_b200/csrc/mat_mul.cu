@@ -64,7 +64,7 @@ static int run_skinny(const rg_mat_mul_params *p, void *ws, const void *const *i
 // and 0.83 per 16 values
 static float f32_simt_us(const rg_mat_mul_params *p) {
     const float tiles = static_cast<float>((p->m + 63) / 64) * static_cast<float>((p->n + 63) / 64) * static_cast<float>(p->batch);
-    const float steps = static_cast<float>((p->k + 15) / 16), alone = 1.48f * steps, full = tiles / static_cast<float>(sm_count()) * (0.3f + 0.83f * steps);
+    const float steps = p->k > 16 ? static_cast<float>(p->k) / 16.f : 1.f, alone = 1.48f * steps, full = tiles / static_cast<float>(sm_count()) * (0.3f + 0.83f * steps);
     return 3.f + (alone > full ? alone : full);
 }
 // fp32 (force_kernel values): the form with the smallest estimated time.  Measured (tensor cores / 32 x 32 tiles / 64 x 64 tiles):
