@@ -1,6 +1,7 @@
 // General MatMul on CUDA cores: any transpose combination, batch strides with broadcast, bias, alpha/beta,
 // fp32 accumulation.  This is the catch-all behind rg_b200_mat_mul (MatMulInfo semantics,
-// src/04kernel/src/attributes/mat_mul_info.cc:27-42) and takes what the tcgen05, streaming and 32 x 32 fp32 kernels do not.
+// src/04kernel/src/attributes/mat_mul_info.cc:27-42) and takes what the tcgen05, streaming and 32 x 32 fp32 kernels do not, and fp32
+// results with a short k.
 #include "common.cuh"
 #include "gemm_dispatch.cuh"
 

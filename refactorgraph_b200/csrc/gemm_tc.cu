@@ -14,7 +14,8 @@
 // The accumulator is double-buffered in tensor memory (2 x BN columns, acc_full[] / acc_empty[] mbarriers), so a tile's
 // epilogue overlaps the next tile's main loop.  Warp 5 also allocates and frees the TMEM columns.  Every mbarrier wait is bounded; on expiry the CTA records
 // an error word, still frees its tensor memory and exits.
-// Products of 512 rows and more run on CTA pairs (template flag PAIR, tcgen05 ... cta_group::2): see the comment above the kernel.
+// Large products (512 rows and more, where tc_wide_tile says so) run on CTA pairs (template flag PAIR, tcgen05 ... cta_group::2): see
+// the comment above the kernel.
 #include "gemm_dispatch.cuh"
 #include "tcgen05.cuh"
 #include "ar_slots.cuh"
@@ -655,7 +656,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             // tile of 128 x 256 took 12 us longer than the plain product with a load in front of every store.
             // Rows of a multiple of 8 columns end between two 16-byte pieces, which are then there or not, and past the last column there is
             // nothing to do: straight-line code for single columns costs more than its stores when it comes from a cold instruction cache
-            // (128 x 64 x 64 7.5 us with it, 1945 x 8040 x 312 33.4).
+            // (128 x 64 x 64 7.5 us with it and 2.9 without, 1945 x 8040 x 312 33.4 and 24.4).
             const bool rows_wide = a.y_col_stride == 1 && (a.n % 8) == 0 && (a.y_row_stride % 8) == 0 && (!C || c_rowmajor);
             Vec16<T> cnext[4];
             auto fetch_c = [&](uint32_t col0) {

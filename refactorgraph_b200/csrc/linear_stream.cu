@@ -409,7 +409,7 @@ using namespace rg;
 extern "C" {
 // 5..32 tokens without a norm prologue: the skinny weight-streaming kernel (linear_skinny.cu)
 // SiLU gate on 5..64 tokens: the tcgen05 kernel with the weights on the M side, except for the few-rows / long-k shape the
-// streaming skinny kernel is faster on (the rule of the plain product)
+// streaming skinny kernel is faster on
 static bool linear_is_tc_swiglu_small(const rg_linear_params *p) {
     if (!gemm_tc_swiglu_small_shape(p)) return false;
     const bool skinny_wins = p->m <= 16 && p->n <= 2560 && p->k >= 4096 && linear_skinny_shape(p->dtype, p->m, p->n, p->k);

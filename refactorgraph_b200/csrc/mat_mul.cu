@@ -71,7 +71,7 @@ static float f32_simt_us(const rg_mat_mul_params *p) {
 // 32 x 256 x 256 9.0 / 4.1 / 18.2 us, 128 x 1024 x 1024 19.7 / 19.0 / 97.8, 256 x 1024 x 1024 20.1 / 19.3 / -, 32 x 32000 x 1024 49 / 66 / 295,
 // 4 x 11008 x 4096 75 / 103 / -, 509 x 2752 x 1024 39 / 91 / 128; the 64 x 64 tiles have the short k of large results, where the others pay
 // for every tile: 4096 x 4096 x 4 - / 111 / 34, 1024 x 1024 x 8 - / 8.5 / 3.9, 300 matrices of 100 x 100 x 10 - / 31 / 11, 512 of 64 x 64 x 64
-// - / 18.1 / 14.6.
+// - / 18.1 / 14.6.  Sums of fewer than eight products stay off the tensor cores, whose dropped terms would show beside so few roundings.
 static int f32_route(const rg_mat_mul_params *p) {
     if (p->trans_a || !gemm_small32_supported(p)) return p->trans_a ? 1 : 5;
     const float tc = p->k < 8 ? 1e30f : gemm_tc32_us(p), small = gemm_small32_us(p);
